@@ -134,6 +134,35 @@ static __device__ __noinline__ void count_wait(volatile int* word, int want,
   }
 }
 
+// A wait by a whole converged warp: the vote makes the branch uniform, so that the common case is
+// three instructions.
+__device__ __forceinline__ void mbar_wait_warp(uint32_t bar, uint32_t parity,
+                                               volatile int* abort_flag, int* status) {
+  if (!__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) {
+    mbar_wait_slow(bar, parity, abort_flag, status);
+    __syncwarp();
+  }
+}
+// One arrival for a converged warp, by an elected lane (no branch).
+__device__ __forceinline__ void mbar_arrive_elect(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xFFFFFFFF;\n\t"
+      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar) : "memory");
+}
+// Arrival at a named barrier without waiting there.
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c,
+                                             uint32_t d) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void ld_shared_f4(uint32_t addr, float& a, float& b, float& c, float& d) {
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(a), "=f"(b), "=f"(c), "=f"(d) : "r"(addr));
+}
+
 // Bounded wait that ignores the abort flag: used once, at exit, to let a CTA's own bulk copies
 // land before its shared memory is released.
 __device__ inline void mbar_wait_drain(uint32_t bar, uint32_t parity, long long budget) {
@@ -278,6 +307,52 @@ __device__ inline void umma_ts_c(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo
       "setp.ne.b32 p, %5, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], db, %4, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "n"(B_HI), "n"(IDESC), "n"(ACC ? 1 : 0)
+      : "memory");
+}
+
+// Four chained MMAs issued by an elected lane of a converged warp: D starts at zero; the K steps
+// advance A by eight tensor-memory columns (or A_STEP descriptor units) and B by 32 bytes (or
+// B_STEP). The tensor-memory form ends with the commit that arrives on `bar`.
+template <uint32_t B_HI, uint32_t IDESC>
+__device__ __forceinline__ void umma_ts_chain4(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e, z, o;\n\t.reg .b64 b0, b1, b2, b3;\n\t"
+      "elect.sync _|e, 0xFFFFFFFF;\n\t"
+      "setp.ne.b32 z, 0, 0;\n\tsetp.eq.b32 o, 0, 0;\n\t"
+      "mov.b64 b0, {%4, %8};\n\tmov.b64 b1, {%5, %8};\n\t"
+      "mov.b64 b2, {%6, %8};\n\tmov.b64 b3, {%7, %8};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], b0, %9, z;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%2], b1, %9, o;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%3], b2, %9, o;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%10], b3, %9, o;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t}"
+      ::"r"(d), "r"(a), "r"(a + 8), "r"(a + 16), "r"(b_lo), "r"(b_lo + 2), "r"(b_lo + 4),
+        "r"(b_lo + 6), "n"(B_HI), "n"(IDESC), "r"(a + 24), "r"(bar)
+      : "memory");
+}
+template <uint32_t A_HI, uint32_t B_HI, uint32_t IDESC, uint32_t A_STEP, uint32_t B_STEP>
+__device__ __forceinline__ void umma_ss_chain4(uint32_t d, uint32_t a_lo, uint32_t b_lo) {
+  asm volatile(
+      "{\n\t.reg .pred e, z, o;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t"
+      "elect.sync _|e, 0xFFFFFFFF;\n\t"
+      "setp.ne.b32 z, 0, 0;\n\tsetp.eq.b32 o, 0, 0;\n\t"
+      "mov.b64 a0, {%1, %9};\n\tmov.b64 a1, {%2, %9};\n\t"
+      "mov.b64 a2, {%3, %9};\n\tmov.b64 a3, {%4, %9};\n\t"
+      "mov.b64 b0, {%5, %10};\n\tmov.b64 b1, {%6, %10};\n\t"
+      "mov.b64 b2, {%7, %10};\n\tmov.b64 b3, {%8, %10};\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a0, b0, %11, z;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a1, b1, %11, o;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a2, b2, %11, o;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a3, b3, %11, o;\n\t}"
+      ::"r"(d), "r"(a_lo), "r"(a_lo + A_STEP), "r"(a_lo + 2 * A_STEP), "r"(a_lo + 3 * A_STEP),
+        "r"(b_lo), "r"(b_lo + B_STEP), "r"(b_lo + 2 * B_STEP), "r"(b_lo + 3 * B_STEP), "n"(A_HI),
+        "n"(B_HI), "n"(IDESC)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_elect(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
       : "memory");
 }
 

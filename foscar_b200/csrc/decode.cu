@@ -19,8 +19,8 @@
 //                 into S row t, joins the group's column max, writes its P row; one tile later
 //                 thread d adds channel d of the tile's O to the group's accumulators. Each
 //                 group keeps its own running (m, l, c, O); they are merged once per work item.
-//   warp 17       S issuer (one thread):  S[128 tok x 16] = C_K . Q^T   (A from tensor memory)
-//   warp 18       PV issuer (one thread): O^T[128 ch x 16] = C_V^T . [P_hi | P_lo]
+//   warp 17       S issuer:  S[128 tok x 16] = C_K . Q^T   (A from tensor memory)
+//   warp 18       PV issuer: O^T[128 ch x 16] = C_V^T . [P_hi | P_lo]
 //
 // Why one group per tile rather than a role per stage: the kernel is bound by instruction issue
 // and by hand-off latency, not by arithmetic. With separate unpack and softmax roles every tile
@@ -28,8 +28,18 @@
 // arithmetic removed, that skeleton alone took 70% of the launch time. Here a tile costs each of
 // its four warps three waits (codes landed, S done, previous PV done) and three arrivals, the
 // group's K stage, S, V stage, P rows and O need no barrier of their own (the group itself was
-// their last reader), and a group's chain of dependent latencies (~1500-2000 cycles a tile)
+// their last reader), and a group's chain of dependent latencies (~2600 cycles a tile)
 // overlaps with the other three groups'.
+// The hand-offs are kept to few instructions: every role runs as whole converged warps, waits vote
+// so that their branch is uniform, single-lane work (arrivals, MMAs, commits) is predicated by
+// elect.sync inside one asm block, ring stages and barriers sit at compile-time offsets, and values
+// that are the same in a warp are told to the compiler (uniform()), because tensor-memory, barrier
+// and descriptor operands have to be in uniform registers. A tile took 1930 warp instructions with
+// lane-0 branches and run-time offsets and takes 1490; on one box 32 requests of 4K-32K tokens (INT2,
+// 32/8 heads) went from 107.8 to 97.4 us, 16 requests of 16K with two query tokens from 66.7 to
+// 55.7, the head_dim 64 build on 256 requests of 64-131072 tokens from 707 to 595. Three, five and
+// six groups measure the same or slower (the registers they cost), and so does one MMA in place of a
+// chain of four: what is left is the instructions' own latency at five warps a scheduler.
 // Every role walks the same list of work items, so the pipeline never drains inside an item.
 // Byte-expansion yields channels in a fixed permuted order; Q is loaded in that order and O is
 // stored through it, so no per-element fix-up exists anywhere.
@@ -47,102 +57,57 @@
 // unit's counter one tile into the CTA's next item (or after its last), once every worker warp
 // has reported its stores of the piece on a barrier, and the CTA that completes the count merges
 // the unit (merge_unit_partials).
-// The ring's stage count is kept even, so that each stage belongs to one of the two producers.
+// The ring's stage count is even, so that each stage belongs to one of the two producers.
 #include "decode.cuh"
-
-#ifdef FQ_WAIT_PROFILE
-#define FQ_STAMP_BEGIN() long long stamp_t = clock64()
-#define FQ_STAMP(site)                                            \
-  do {                                                            \
-    const long long now_ = clock64();                             \
-    wprof[site] += static_cast<int>(now_ - stamp_t);              \
-    stamp_t = now_;                                               \
-  } while (0)
-#define FQ_ITEM_STAMP_BEGIN() long long item_t = clock64()
-#define FQ_ITEM_STAMP(site)                                       \
-  do {                                                            \
-    const long long now_ = clock64();                             \
-    wprof[site] += static_cast<int>(now_ - item_t);               \
-    item_t = now_;                                                \
-  } while (0)
-#else
-#define FQ_STAMP_BEGIN() ((void)0)
-#define FQ_STAMP(site) ((void)0)
-#define FQ_ITEM_STAMP_BEGIN() ((void)0)
-#define FQ_ITEM_STAMP(site) ((void)0)
-#endif
-
-// Diagnostic builds only: a bit mask of roles whose arithmetic is skipped while every barrier
-// arrival stays (1 softmax, 2 K unpack, 4 V unpack, 8 producers' copies; 16 / 32: one S / PV MMA
-// per tile instead of four; 64 / 128: the INT2 K / V unpack at the instruction count of a 4-bit
-// operand feed, i.e. two masks and a shift per packed word and half the operand words stored,
-// at head_dim 128; 256 / 512: one of a row's eight V operand stores / four K operand stores
-// only). The output is
-// then meaningless; the launch time and instruction count show what each role costs.
-#ifndef FQ_STUB_ROLES
-#define FQ_STUB_ROLES 0
-#endif
 
 namespace fq {
 
-#ifdef FQ_WAIT_PROFILE
-// Diagnostic build only: per-CTA cycles (/16) each role spent blocked at each wait site.
-__device__ int* g_wait_profile = nullptr;
-#endif
-
 namespace {
 
-// barrier words: the ring's 2*ns first, then the fixed ones
-template <int G>
+// Barrier words of a CTA, at fixed offsets: one per ring stage and direction, one per query stage
+// and direction, and per worker group
+//   s_done  : the tile's S MMA is complete (commit)
+//   pv_ready: the tile's V operand and P rows are in shared memory (the group's four warps); the
+//             group has by then read the O of its previous tile
+//   pv_done : the tile's PV MMA is complete (commit): O can be read, and the group's V stage and P
+//             rows are free
+// A group's n-th tile uses phase n & 1. stored: every worker warp has issued its output or partial
+// stores of the work item (one phase per item): what orders a split piece's partials before its
+// count-in. That a group's K operand is in tensor memory goes from its four warps to the S issuer
+// through a named barrier of 160 threads (K_READY): one instruction a warp.
+template <int G, int NS>
 struct Bars {
   uint32_t base;
-  int ns;
-  __device__ uint32_t at(int i) const { return base + 8u * i; }
-  __device__ uint32_t ring_full(int s) const { return at(s); }
-  __device__ uint32_t ring_empty(int s) const { return at(ns + s); }
-  __device__ uint32_t q_full(int s) const { return at(2 * ns + s); }
-  __device__ uint32_t q_empty(int s) const { return at(2 * ns + 2 + s); }
-  // One barrier per worker group and event; a group's n-th tile uses phase n & 1:
-  //   k_ready : the tile's K operand is in tensor memory (the group's 4 warps); the group has by
-  //             then read the S of its previous tile
-  //   s_done  : the tile's S MMA is complete (commit)
-  //   pv_ready: the tile's V operand and P rows are in shared memory (4 warps); the group has by
-  //             then read the O of its previous tile
-  //   pv_done : the tile's PV MMA is complete (commit): O can be read, and the group's V stage
-  //             and P rows are free
-  __device__ uint32_t k_ready(int g) const { return at(2 * ns + 4 + g); }
-  __device__ uint32_t s_done(int g) const { return at(2 * ns + 4 + G + g); }
-  __device__ uint32_t pv_ready(int g) const { return at(2 * ns + 4 + 2 * G + g); }
-  __device__ uint32_t pv_done(int g) const { return at(2 * ns + 4 + 3 * G + g); }
-  // stored: every worker warp has issued its output or partial stores of the work item (one
-  // phase per item): what orders a split piece's partials before its count-in
-  __device__ uint32_t stored() const { return at(2 * ns + 4 + 4 * G); }
-  // 2*ns + 5 + 4*G words of 8 bytes
+  __device__ uint32_t ring_full(int s) const { return base + 8u * s; }
+  __device__ uint32_t ring_empty(int s) const { return base + 8u * (NS + s); }
+  __device__ uint32_t q_full(int s) const { return base + 8u * (2 * NS + s); }
+  __device__ uint32_t q_empty(int s) const { return base + 8u * (2 * NS + 2 + s); }
+  __device__ uint32_t s_done(int g) const { return base + 8u * (2 * NS + 4 + g); }
+  __device__ uint32_t pv_done(int g) const { return base + 8u * (2 * NS + 4 + G + g); }
+  __device__ uint32_t pv_ready(int g) const { return base + 8u * (2 * NS + 4 + 2 * G + g); }
+  __device__ uint32_t stored() const { return base + 8u * (2 * NS + 4 + 3 * G); }
+  static constexpr int WORDS = 2 * NS + 5 + 3 * G;
 };
-
-// Position in the code ring: stage and phase, advanced without a division.
-struct RingPos {
-  int s = 0;
-  uint32_t ph = 0;
-  __device__ __forceinline__ void next(int ns) {
-    if (++s == ns) { s = 0; ph ^= 1u; }
-  }
-  __device__ __forceinline__ void advance(int k, int ns) {  // k <= ns
-    s += k;
-    if (s >= ns) { s -= ns; ph ^= 1u; }
-  }
-};
+// Named barriers: 0 the CTA, 1 .. G inside a group, 1 + G all groups, then one per group for its K
+// operand (there are sixteen in all).
+template <int G> constexpr int K_READY = 2 + G;
 
 // Tensor-memory column plan (f32 columns): per worker group one K operand stage (a 128-byte row
-// per lane at head_dim 64, where a lane holds two tokens), one S buffer of 16 columns and one O
-// buffer of 16 columns per token of a lane.
+// per lane; at head_dim 64 a lane holds two tokens), one S buffer of 16 columns and one O buffer
+// of 16 columns per token of a lane.
+// INT2 with whole-head K at head_dim 128: the K rows are unpacked like the V rows, at five instead
+// of seven instructions a packed word (odd operand words hold 4 * code), and the idle half of the
+// sixteen query rows takes the odd words' products into score columns 8-15.
+__host__ __device__ constexpr bool odd_columns(int bits, int head_dim, int kg) {
+  return bits == 2 && head_dim == 128 && kg != 2;
+}
+
 template <int BITS, int D>
 struct TmemPlan {
   static constexpr int G = worker_groups(BITS, D);
   static constexpr bool PAIR = D == 64;
-  static constexpr bool TWO = two_token_build(BITS, D);   // two 128-byte rows, two S buffers
-  static constexpr int KOP_COLS = PAIR ? 32 : (TWO ? 2 : 1) * D / 4;
-  static constexpr int S_COLS = TWO ? 32 : 16;
+  static constexpr int KOP_COLS = 32;
+  static constexpr int S_COLS = 16;
   static constexpr int O_COLS = PAIR ? 32 : 16;
   static constexpr int KOP = 0;
   static constexpr int S = G * KOP_COLS;
@@ -152,63 +117,55 @@ struct TmemPlan {
   static_assert(USED <= 512, "tensor memory plan exceeds 512 columns");
 };
 
-// Worker role: one of four 128-thread groups. Group `wg` takes the tiles whose running index is
-// `wg` modulo 4 and carries each of them through every stage itself: unpack K into tensor memory,
-// unpack V into shared memory, fold the scales into the raw scores, softmax, write the P rows,
-// and (one of its own tiles later) add the tile's O to its accumulators. The group keeps its own
-// running (m, l, c, O); the four groups are merged once per work item.
 // The request's last tile with several query tokens per request: column h sees positions below
 // len - lag(h) only. Out of line, so that this rare path (and column_lag's division) costs the
 // tile loop nothing: the scores pass through local memory here and nowhere else. `pos0` is the
 // thread's first token position of the tile, `stride` the distance to its next one. Returns,
-// in `over`, the largest excess of a visible score over its column's reference.
+// in `over`, the largest visible score.
 template <int NT, int GP>
 __device__ __noinline__ void mask_lagged_columns(const DecodeParams& P, int len, int ht, int pos0,
-                                                 int stride, float (&x)[NT][GP],
-                                                 const float (&m)[GP], float& over) {
+                                                 int stride, float (&x)[NT][GP], float& over) {
   float top = -INFINITY;
   for (int h = 0; h < GP; ++h) {
     const int lim = len - column_lag(P, ht * 8 + h);
     for (int u = 0; u < NT; ++u) {
       if (pos0 + u * stride >= lim) x[u][h] = -INFINITY;
-      top = fmaxf(top, x[u][h] - m[h]);
+      top = fmaxf(top, x[u][h]);
     }
   }
   over = top;
 }
 
+// Worker role: one of four 128-thread groups. Group `wg` takes the tiles whose running index is
+// `wg` modulo 4 and carries each of them through every stage itself: unpack K into tensor memory,
+// unpack V into shared memory, fold the scales into the raw scores, softmax, write the P rows,
+// and (one of its own tiles later) add the tile's O to its accumulators. The group keeps its own
+// running (m, l, c, O); the four groups are merged once per work item.
 template <int BITS, int D, int GP, int KG, bool MQ>
 __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem, uint32_t smem0,
-                                            uint32_t tmem, const Bars<SmemPlan<BITS, D>::G>& bars,
-                                            volatile int* abort_flag, const ItemRange items,
-                                            int* wprof) {
+                                            uint32_t tmem,
+                                            const Bars<SmemPlan<BITS, D>::G, SmemPlan<BITS, D>::NS>& bars,
+                                            volatile int* abort_flag, const ItemRange items) {
   using SP = SmemPlan<BITS, D>;
   using TP = TmemPlan<BITS, D>;
-  constexpr int G = SP::G;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int G = SP::G, NS = SP::NS;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int wg = warp >> 2, wq = warp & 3;
   const int t = threadIdx.x & 127;  // token row while unpacking and in softmax, channel in O
-  const int NS = P.ring_stages;
   int* status = P.a.status;
   const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
-  const uint32_t ring0 = smem0 + SP::RING_OFF;
   const uint32_t k_dst = tmem + lane_base + TP::KOP + wg * TP::KOP_COLS;
   const uint32_t s_src = tmem + lane_base + TP::S + wg * TP::S_COLS;
   constexpr int NT = SP::TT / TILE;   // tokens per lane
+  constexpr bool ODD = odd_columns(BITS, D, KG);
   // a lane's O columns: at two tokens per lane, rows 0-63 (warps 0, 1) hold the first token
   // set's channels and take its P columns, rows 64-127 the second's
   const uint32_t o_src = tmem + lane_base + TP::O + wg * TP::O_COLS + (SP::PAIR && wq >= 2 ? 16 : 0);
-  const uint32_t v_row = smem0 + SP::VOP_OFF + wg * SP::VOP_STAGE + t * SP::ROW;
+  // (rows are 128 bytes at a 1024-byte aligned base: piece cc of the swizzled row is an xor away)
+  const uint32_t v_row = (smem0 + SP::VOP_OFF + wg * SP::VOP_STAGE + t * SP::ROW) | ((t & 7) << 4);
   const uint32_t p_row = smem0 + SP::P_OFF + wg * SP::P_BYTES + t * 16;
-#if FQ_STUB_ROLES & (64 | 128)
-  {   // the operand words the short stubs never write: zero once
-    uint32_t zero[8] = {};
-    for (int v = 0; v < TP::KOP_COLS / 8; ++v) tmem_st8(k_dst + 8 * v, zero);
-    tmem_st_wait();
-    for (int cc = 0; cc < 8; ++cc)
-      asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(v_row + (cc << 4)), "r"(0) : "memory");
-  }
-#endif
+  // the thread's code row in a ring stage, at its piece 0: piece v is an xor away
+  const uint32_t code_row = t * SP::RB + (SP::row_swizzle(t) << 4);
   float* red_max = reinterpret_cast<float*>(smem + SP::RED_OFF);              // [wg][buf][warp][8]
   float* red_sum = reinterpret_cast<float*>(smem + SP::RED_OFF + 256 * G);    // [wg][warp][16]
   // this warp's copy of the item's per-head constants: sm_scale*log2e*q_descale, and that times
@@ -236,7 +193,7 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
     lp = 135 - max(top, 27);
   }
   // w = p * s_v * 2^lp must stay inside E4M3 with p up to 2^MAX_LAG (see the softmax below)
-  constexpr float MAX_LAG = 3.f;
+  constexpr float MAX_LAG = 3.f, HEADROOM = 3.f;
   lp -= static_cast<int>(MAX_LAG);
   const float p2lp = exp2f(static_cast<float>(lp));
   const float o_mul = exp2f(static_cast<float>(9 - lp));
@@ -250,25 +207,35 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
   int pend_k = 0, pend_unit = 0, pend_b = 0, pend_kvh = 0, pend_ht = 0;
   uint32_t pend_phase = 0;   // phase of the `stored` barrier that covers the pending piece
   int seen = -1;        // the pending piece's count-in result; -1: not counted in yet
+  bool count_due = false;    // (warp 0) a piece is pending and not counted in
   int this_k = 0;       // pieces of the current item's unit (fetched at the item's start)
+  auto count_in = [&]() {
+    count_due = false;
+    if (lane == 0) {
+      mbar_wait(bars.stored(), pend_phase, abort_flag, status);
+      __threadfence();
+      seen = atomicAdd(P.a.unit_counters + pend_unit, 1);
+    }
+    __syncwarp();
+  };
 
   int qi = 0;       // non-empty items so far: which query stage holds the item's rows
   int it0 = 0;      // running index of the current item's first tile (every role counts alike)
   int mine = wg;    // running index of this group's next tile
-  int n = 0;        // tiles this group has taken: the phase of its barriers
-  RingPos rp;       // ring position of tile `mine`
-  rp.advance(wg, NS);
-  FQ_ITEM_STAMP_BEGIN();
+  uint32_t ph = 0;  // phase of the group's barriers: flips with every tile
+  // ring position of tile `mine`
+  uint32_t stage = smem0 + SP::RING_OFF + wg * SP::STAGE;
+  uint32_t full = bars.ring_full(wg), ring_ph = 0;
   const WorkItem* const item_cache = reinterpret_cast<const WorkItem*>(smem + SP::ITEM_OFF);
   const WorkItem* const item_more =
       reinterpret_cast<const WorkItem*>(smem + SP::RING_OFF + NS * SP::STAGE);
   for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
-    const WorkItem w = item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi);
+    const WorkItem w = uniform_item(item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi));
     const int nt = max(w.t1 - w.t0, 0);
-    FQ_ITEM_STAMP(13);
     float m[GP], l[GP], c[GP], oacc[GP];
 #pragma unroll
-    for (int h = 0; h < GP; ++h) { m[h] = -INFINITY; l[h] = 0.f; c[h] = 0.f; oacc[h] = 0.f; }
+    for (int h = 0; h < GP; ++h) { m[h] = 0.f; l[h] = 0.f; c[h] = 0.f; oacc[h] = 0.f; }
+    uint32_t unset = (1u << GP) - 1u;   // heads without a finite score so far: m is no reference
     // The item's per-head constants (score scale, and score scale times the sum of the head's
     // query values) were computed by the first producer when it staged the query rows, well
     // ahead of the tiles; the warp keeps its own copy, read back from shared memory each tile
@@ -281,7 +248,7 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       // stagings behind never returns.
       if (mine < it0 + nt) {
         const int qb = qi & 1;
-        mbar_wait(bars.q_full(qb), (qi >> 1) & 1, abort_flag, status, 14, wprof);
+        mbar_wait(bars.q_full(qb), (qi >> 1) & 1, abort_flag, status);
         if (lane < 24) head_k[lane] = head_const[qb * 24 + lane];
       }
       ++qi;
@@ -292,167 +259,71 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       const int unit = (w.b * P.p.num_kv_heads + w.kvh) * P.head_tiles + w.ht;
       this_k = P.a.split_counts != nullptr ? __ldg(P.a.split_counts + unit) : P.a.kv_splits;
     }
-    FQ_ITEM_STAMP(16);
 
     // Add the group's previous tile's O (its PV MMA has had most of a tile's time to finish).
     // The wait also frees the group's V stage and P rows for the tile in hand.
     auto accumulate = [&]() {
-      mbar_wait(bars.pv_done(wg), (n - 1) & 1, abort_flag, status, 15, wprof);
+      mbar_wait_warp(bars.pv_done(wg), ph ^ 1u, abort_flag, status);
       tc_fence_after();
       uint32_t r[16];
       tmem_ld16(o_src, r);
       tmem_ld_wait();
-      tc_fence_before();
 #pragma unroll
       for (int h = 0; h < GP; ++h)
         oacc[h] += fmaf(__uint_as_float(r[8 + h]), 0.0625f, __uint_as_float(r[h]));
     };
 
-    for (; mine < it0 + nt; mine += G, rp.advance(G, NS), ++n) {
-      const int tt = w.t0 + (mine - it0);
-      const uint32_t stage = ring0 + rp.s * SP::STAGE;
-      mbar_wait(bars.ring_full(rp.s), rp.ph, abort_flag, status, 8, wprof);
-      FQ_STAMP_BEGIN();
+    // first position of the thread's row in the group's next tile; tiles up to `whole` lie
+    // entirely inside what every column sees
+    int pos0 = (w.t0 + (mine - it0)) * SP::TT + t;
+    const int whole = w.len - (MQ ? P.q_len - 1 : 0) - SP::TT + t;
+#pragma unroll 1
+    for (; mine < it0 + nt; mine += G, pos0 += G * SP::TT) {
+      mbar_wait_warp(full, ring_ph, abort_flag, status);
       // ---- K row(s) -> tensor memory (the S MMA's A operand). The stage is free: this group
       // read the S of its previous tile, so that tile's MMA, the stage's last reader, is
       // complete. With two tokens per lane (head_dim 64) the second token's 64 bytes follow the
       // first's in the lane's 128-byte row.
-      {
-        if constexpr (SP::PAIR) {
-          // Two tokens per lane: one token's row (64 channels, 16 operand words) at a time, in a
-          // loop that is NOT unrolled. This build's tile loop is the largest, and with the loop
-          // rolled its code stays in the instruction cache better (INT4 838 -> 819 us on C5;
-          // the same rolling at head_dim 128 cost 2 to 9 %).
-          constexpr int QC = 64 * BITS / 128;   // 16-byte chunks of a token's row: 1 or 2
-          tc_fence_after();
+      if constexpr (SP::PAIR) {
 #pragma unroll 1
-          for (int u = 0; u < 2; ++u) {
-            uint32_t wk[64 * BITS / 32], op[16];
-#if FQ_STUB_ROLES & 2
-#pragma unroll
-            for (int i = 0; i < 16; ++i) op[i] = n;
-#else
-            const uint32_t row = stage + SP::K_OFF + (u * TILE + t) * SP::RB;
-#pragma unroll
-            for (int v = 0; v < QC; ++v)
-              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(wk[4 * v]), "=r"(wk[4 * v + 1]), "=r"(wk[4 * v + 2]),
-                             "=r"(wk[4 * v + 3])
-                           : "r"(row + ((v ^ SP::row_swizzle(t)) << 4)));
-            expand_words<BITS, 64>(wk, op);
-#endif
-            tmem_st16(k_dst + 16 * u, op);
-          }
-          FQ_STAMP(3);
-        } else {
-          uint32_t op[NT * D / 4];
-#pragma unroll
-          for (int u = 0; u < NT; ++u) {
-            uint32_t wk[D * BITS / 32], part[D / 4];
-#if FQ_STUB_ROLES & 2
-#pragma unroll
-            for (int i = 0; i < D / 4; ++i) part[i] = n;
-#else
-            load_row<BITS, D>(stage + SP::K_OFF + (u * TILE + t) * SP::RB, wk, SP::row_swizzle(t));
-#if FQ_STUB_ROLES & 64
-            if constexpr (BITS == 2) {
-#pragma unroll
-              for (int i = 0; i < D / 16; ++i) {
-                part[2 * i] = wk[i] & 0x33333333u;
-                part[2 * i + 1] = (wk[i] >> 2) & 0x33333333u;
-              }
-            } else
-#endif
-            expand_words<BITS, D>(wk, part);
-#endif
-#pragma unroll
-            for (int i = 0; i < D / 4; ++i) op[u * (D / 4) + i] = part[i];
-          }
-          FQ_STAMP(3);
-          tc_fence_after();
-#pragma unroll
-          for (int v = 0; v < NT * D / (((FQ_STUB_ROLES & 64) && BITS == 2) ? 64 : 32); ++v)
-            if (!(FQ_STUB_ROLES & 512) || v == 0) tmem_st8(k_dst + 8 * v, op + 8 * v);
+        for (int u = 0; u < 2; ++u) {
+          uint32_t wk[64 * BITS / 32], op[16];
+          load_code_row<BITS, 64>(stage + SP::K_OFF + u * TILE * SP::RB + code_row, wk);
+          expand_words<BITS, 64>(wk, op);
+          tmem_st16(k_dst + 16 * u, op);
         }
-        tmem_st_wait();
-        FQ_STAMP(5);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bars.k_ready(wg));
+      } else {
+        uint32_t wk[D * BITS / 32], op[D / 4];
+        load_code_row<BITS, D>(stage + SP::K_OFF + code_row, wk);
+        if constexpr (ODD) expand_words_v<BITS, D>(wk, op);
+        else expand_words<BITS, D>(wk, op);
+        tmem_st32(k_dst, op);
       }
-      FQ_STAMP(17);
+      tmem_st_wait();
+      tc_fence_before();
+      named_arrive(K_READY<G> + wg, 160);
       if (pending) accumulate();
-      FQ_STAMP(18);
       // ---- V row(s) -> the group's 128-byte-swizzled shared-memory stage (the PV MMA's A
       // operand), laid out like the K row
       if constexpr (SP::PAIR) {
-        constexpr int QC = 64 * BITS / 128;
 #pragma unroll 1
         for (int u = 0; u < 2; ++u) {
           uint32_t wv[64 * BITS / 32], op[16];
-#if FQ_STUB_ROLES & 4
-#pragma unroll
-          for (int i = 0; i < 16; ++i) op[i] = n;
-#else
-          const uint32_t row = stage + SP::V_OFF + (u * TILE + t) * SP::RB;
-#pragma unroll
-          for (int v = 0; v < QC; ++v)
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(wv[4 * v]), "=r"(wv[4 * v + 1]), "=r"(wv[4 * v + 2]),
-                           "=r"(wv[4 * v + 3])
-                         : "r"(row + ((v ^ SP::row_swizzle(t)) << 4)));
+          load_code_row<BITS, 64>(stage + SP::V_OFF + u * TILE * SP::RB + code_row, wv);
           expand_words_v<BITS, 64>(wv, op);
-#endif
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
-                             v_row + (((4 * u + cc) ^ (t & 7)) << 4)),
-                         "r"(op[4 * cc]), "r"(op[4 * cc + 1]), "r"(op[4 * cc + 2]),
-                         "r"(op[4 * cc + 3])
-                         : "memory");
-          }
+          for (int cc = 0; cc < 4; ++cc)
+            st_shared_v4((v_row ^ (u << 6)) ^ (cc << 4), op[4 * cc], op[4 * cc + 1], op[4 * cc + 2],
+                         op[4 * cc + 3]);
         }
-        FQ_STAMP(6);
       } else {
-        uint32_t op[NT * D / 4];
+        uint32_t wv[D * BITS / 32], op[D / 4];
+        load_code_row<BITS, D>(stage + SP::V_OFF + code_row, wv);
+        expand_words_v<BITS, D>(wv, op);
 #pragma unroll
-        for (int u = 0; u < NT; ++u) {
-          uint32_t wv[D * BITS / 32], part[D / 4];
-#if FQ_STUB_ROLES & 4
-#pragma unroll
-          for (int i = 0; i < D / 4; ++i) part[i] = n;
-#else
-          load_row<BITS, D>(stage + SP::V_OFF + (u * TILE + t) * SP::RB, wv, SP::row_swizzle(t));
-#if FQ_STUB_ROLES & 128
-          if constexpr (BITS == 2) {
-#pragma unroll
-            for (int i = 0; i < D / 16; ++i) {
-              part[2 * i] = wv[i] & 0x33333333u;
-              part[2 * i + 1] = (wv[i] >> 2) & 0x33333333u;
-            }
-          } else
-#endif
-          expand_words_v<BITS, D>(wv, part);
-#endif
-#pragma unroll
-          for (int i = 0; i < D / 4; ++i) op[u * (D / 4) + i] = part[i];
-        }
-        FQ_STAMP(6);
-#pragma unroll
-        for (int u = 0; u < NT; ++u) {   // token 128 u + t is row 128 u + t of the stage
-#pragma unroll
-          for (int cc = 0; cc < D / (((FQ_STUB_ROLES & 128) && BITS == 2) ? 32 : 16); ++cc) {
-            if ((FQ_STUB_ROLES & 256) && cc > 0) continue;
-            const int oc = u * (D / 16) + cc;
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
-                             v_row + u * TILE * SP::ROW + ((cc ^ (t & 7)) << 4)),
-                         "r"(op[4 * oc]), "r"(op[4 * oc + 1]), "r"(op[4 * oc + 2]),
-                         "r"(op[4 * oc + 3])
-                         : "memory");
-          }
-        }
+        for (int cc = 0; cc < D / 16; ++cc)
+          st_shared_v4(v_row ^ (cc << 4), op[4 * cc], op[4 * cc + 1], op[4 * cc + 2], op[4 * cc + 3]);
       }
-      FQ_STAMP(9);
       // the tokens' records; then the ring stage goes back to the producers
       float sk[NT], zk[NT], sv[NT], zv[NT];
       float sk1[NT] = {}, zk1[NT] = {};   // the second K group's pair (KG == 2)
@@ -482,154 +353,133 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars.ring_empty(rp.s));
-      FQ_STAMP(19);
+      mbar_arrive_elect(full + 8 * NS);   // ring_empty of the stage
+      stage += G * SP::STAGE;
+      full += 8 * G;
+      if (full >= bars.ring_full(NS)) {
+        stage -= NS * SP::STAGE;
+        full -= 8 * NS;
+        ring_ph ^= 1u;
+      }
       // ---- raw scores: columns [0, GP) for the lane's first token, [8, 8 + GP) for its second
-      mbar_wait(bars.s_done(wg), n & 1, abort_flag, status, 12, wprof);
+      mbar_wait_warp(bars.s_done(wg), ph, abort_flag, status);
       tc_fence_after();
-      // (two tokens with a 128-byte row each: a 16-column S buffer per token, RS apart in raw)
-      constexpr int RS = SP::TWO ? (KG == 2 ? 16 : 8) : 8;
-      uint32_t raw[SP::TWO ? 2 * RS : ((NT == 2 || KG == 2) ? 16 : GP)];
-      if constexpr (SP::TWO) {
-        if constexpr (KG == 2) {
-          tmem_ld16p(s_src, raw);
-          tmem_ld16p(s_src + 16, raw + 16);
-        } else {
-          tmem_ld8p(s_src, raw);
-          tmem_ld8p(s_src + 16, raw + 8);
-        }
-      } else if constexpr (NT == 2 || KG == 2) tmem_ld16(s_src, raw);
+      constexpr int RS = 8;
+      uint32_t raw[(NT == 2 || KG == 2 || ODD) ? 16 : GP];
+      if constexpr (NT == 2 || KG == 2 || ODD) tmem_ld16(s_src, raw);
       else if constexpr (GP == 4) tmem_ld4(s_src, raw);
       else tmem_ld8(s_src, raw);
       tmem_ld_wait();
-      tc_fence_before();
-      FQ_STAMP(20);
-      FQ_STAMP(10);   // the cost of one stamp itself
       uint32_t pw[NT][4];
-#if FQ_STUB_ROLES & 1
-#pragma unroll
-      for (int u = 0; u < NT; ++u) {
-        pw[u][0] = __float_as_uint(sk[u] + zk[u]) & 1u; pw[u][1] = raw[0] & 1u;
-        pw[u][2] = __float_as_uint(sv[u] + zv[u]) & 1u; pw[u][3] = 0u;
-      }
-#else
       // Only a request's last tile has positions past its length: their scores become -inf and
       // their records are neutralised, so stale shared memory can never reach the output.
-      // Scores against the group's running reference m, which may lag the true maximum by up to
-      // MAX_LAG (p <= 2^MAX_LAG; the P scale leaves that headroom below the E4M3 range). Only
-      // when some score of the tile exceeds that does the group take the exact column maximum
-      // and rescale; the common tile costs one reducing barrier instead of an exchange through
-      // shared memory.
+      // Scores are taken relative to the group's running reference m, which may lag the true
+      // maximum by up to MAX_LAG (p <= 2^MAX_LAG; the P scale leaves that headroom below the E4M3
+      // range). Only when some score of the tile exceeds that does the group exchange the exact
+      // column maxima and rescale; the common tile costs one reducing barrier.
       float x[NT][GP], wsc[NT];
       float over = -INFINITY;
       // with several query tokens a column stops short of the request's last positions
-      const bool whole = (tt + 1) * SP::TT <= w.len - (MQ ? P.q_len - 1 : 0);
+      const bool inside = pos0 <= whole;   // (the same for the whole group)
+      float hk[GP], hz[GP];
+#pragma unroll
+      for (int h = 0; h < GP; h += 4) {
+        ld_shared_f4(smem_u32(head_k + h), hk[h], hk[h + 1], hk[h + 2], hk[h + 3]);
+        ld_shared_f4(smem_u32(head_k + 8 + h), hz[h], hz[h + 1], hz[h + 2], hz[h + 3]);
+      }
 #pragma unroll
       for (int u = 0; u < NT; ++u) {
-        const int pos = tt * SP::TT + u * TILE + t;
-        const bool valid = whole || pos < w.len;
-        const float a_k = sk[u] * 512.f;
+        const bool valid = inside || pos0 + u * TILE < w.len;
         wsc[u] = sv[u] * p2lp;
         if (!valid) { wsc[u] = 0.f; zv[u] = 0.f; }
 #pragma unroll
         for (int h = 0; h < GP; ++h) {
-          float xv;
+          float xv, s = __uint_as_float(raw[RS * u + h]);
+          if constexpr (ODD) s = fmaf(0.25f, __uint_as_float(raw[8 + h]), s);
           if constexpr (KG == 2)
-            xv = fmaf(head_k[h] * a_k, __uint_as_float(raw[RS * u + h]),
-                      fmaf(head_k[h] * (sk1[u] * 512.f), __uint_as_float(raw[RS * u + 8 + h]),
-                           fmaf(head_k[8 + h], zk[u], head_k[16 + h] * zk1[u])));
+            xv = fmaf(hk[h] * sk[u], s,
+                      fmaf(hk[h] * sk1[u], __uint_as_float(raw[RS * u + 8 + h]),
+                           fmaf(hz[h], zk[u], fmaf(head_k[16 + h], zk1[u], -m[h]))));
           else
-            xv = fmaf(head_k[h] * a_k, __uint_as_float(raw[RS * u + h]), head_k[8 + h] * zk[u]);
+            xv = fmaf(hk[h] * sk[u], s, fmaf(hz[h], zk[u], -m[h]));
           x[u][h] = valid ? xv : -INFINITY;
-          over = fmaxf(over, x[u][h] - m[h]);
+          over = fmaxf(over, x[u][h]);
         }
       }
       if constexpr (MQ) {
-        if (!whole) mask_lagged_columns<NT, GP>(P, w.len, w.ht, tt * SP::TT + t, TILE, x, m, over);
+        if (!inside) mask_lagged_columns<NT, GP>(P, w.len, w.ht, pos0, TILE, x, over);
       }
-      // (a group's first tile of an item always takes the exact maximum: with several query
-      // tokens every score of that tile can be masked, which would leave m at -inf)
-      if (named_barrier_or(1 + wg, 128, over > MAX_LAG || (MQ && m[0] == -INFINITY))) {
-        const int buf = n & 1;
-        float* wmax = red_max + ((wg * 2 + buf) * 4 + wq) * 8;
+      if (named_barrier_or(1 + wg, 128, over > (unset ? -INFINITY : MAX_LAG))) {
+        float* wmax = red_max + ((wg * 2 + ph) * 4 + wq) * 8;
 #pragma unroll
         for (int h = 0; h < GP; ++h) {
           const float wm = warp_max_f32(NT == 2 ? fmaxf(x[0][h], x[NT - 1][h]) : x[0][h]);
           if (lane == 0) wmax[h] = wm;
         }
         named_barrier(1 + wg, 128);
-        const float* gm = red_max + (wg * 2 + buf) * 4 * 8;
+        const float* gm = red_max + (wg * 2 + ph) * 4 * 8;
 #pragma unroll
         for (int h = 0; h < GP; ++h) {
-          // (floored so that a column with every score masked so far has a finite reference)
-          float tm = fmaxf(m[h], fmaxf(fmaxf(gm[h], gm[8 + h]), fmaxf(gm[16 + h], gm[24 + h])));
-          if constexpr (MQ) tm = fmaxf(tm, -1e30f);
-          const float corr = m[h] == -INFINITY ? 0.f : fast_exp2(m[h] - tm);
-          l[h] *= corr;
-          c[h] *= corr;
-          oacc[h] *= corr;   // holds every earlier tile's O (added above)
-          m[h] = tm;
+          const float top = fmaxf(fmaxf(gm[h], gm[8 + h]), fmaxf(gm[16 + h], gm[24 + h]));
+          const bool first = (unset >> h) & 1u;
+          if (top > (first ? -INFINITY : MAX_LAG)) {   // (the same for the whole group)
+            const float delta = top + HEADROOM;
+            // (a head's first reference: its sums are zero)
+            const float corr = first ? 1.f : fast_exp2(-delta);
+            unset &= ~(1u << h);
+            m[h] += delta;
+            l[h] *= corr;
+            c[h] *= corr;
+            oacc[h] *= corr;   // holds every earlier tile's O (added above)
+#pragma unroll
+            for (int u = 0; u < NT; ++u) x[u][h] -= delta;
+          }
         }
       }
-      // two heads per instruction in f16x2: p = 2^(x-m), w = p * s_v 2^lp, E4M3 hi + lo/16
+      // p = 2^x, w = p * s_v 2^lp, four heads at a time as E4M3 hi + lo/16. (ex2 on f32: the
+      // f16x2 form takes twice as long per instruction on this part, so it saves nothing.)
 #pragma unroll
       for (int u = 0; u < NT; ++u) {
-        pw[u][0] = pw[u][1] = pw[u][2] = pw[u][3] = 0u;
-        const __half2 wsc2 = __float2half2_rn(wsc[u]);
 #pragma unroll
-        for (int h = 0; h < GP; h += 2) {
-          const __half2 d2 = __floats2half2_rn(x[u][h] - m[h], x[u][h + 1] - m[h + 1]);
-          const __half2 e2 = h2_exp2(d2);
-          const float2 ef = __half22float2(e2);
-          l[h] += ef.x;
-          l[h + 1] += ef.y;
-          c[h] = fmaf(ef.x, zv[u], c[h]);
-          c[h + 1] = fmaf(ef.y, zv[u], c[h + 1]);
-          const __half2 w2 = __hmul2(e2, wsc2);
-          const uint32_t hi2 = f16x2_to_e4m3x2(w2);
-          const __half2 r2 = __hmul2(__hsub2(w2, e4m3x2_to_f16x2(hi2)), __float2half2_rn(16.f));
-          const uint32_t lo2 = f16x2_to_e4m3x2(r2);
-          pw[u][h >> 2] |= hi2 << (16 * ((h >> 1) & 1));
-          pw[u][2 + (h >> 2)] |= lo2 << (16 * ((h >> 1) & 1));
+        for (int h = 0; h < GP; h += 4) {
+          __half2 w2[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int a = h + 2 * i;
+            const float p0 = fast_exp2(x[u][a]), p1 = fast_exp2(x[u][a + 1]);
+            l[a] += p0;
+            l[a + 1] += p1;
+            c[a] = fmaf(p0, zv[u], c[a]);
+            c[a + 1] = fmaf(p1, zv[u], c[a + 1]);
+            w2[i] = __floats2half2_rn(p0 * wsc[u], p1 * wsc[u]);
+          }
+          split_e4m3x4(w2[0], w2[1], pw[u][h >> 2], pw[u][2 + (h >> 2)]);
         }
+        if constexpr (GP == 4) pw[u][1] = pw[u][3] = 0u;
       }
-#endif
-      FQ_STAMP(21);
       // the P row(s): bytes [hi_0..hi_7 | lo_0..lo_7], one plane of 128 rows per token of a lane;
       // with the V rows above they complete the PV MMA's operands
 #pragma unroll
       for (int u = 0; u < NT; ++u)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(p_row + u * TILE * 16),
-                     "r"(pw[u][0]), "r"(pw[u][1]), "r"(pw[u][2]), "r"(pw[u][3])
-                     : "memory");
+        st_shared_v4(p_row + u * TILE * 16, pw[u][0], pw[u][1], pw[u][2], pw[u][3]);
       fence_proxy_async();
-      FQ_STAMP(11);
+      tc_fence_before();   // (orders the O read above before the PV MMA)
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars.pv_ready(wg));
-      FQ_STAMP(22);
+      mbar_arrive_elect(bars.pv_ready(wg));
       pending = true;
+      ph ^= 1u;
       // The previous split piece of this CTA is counted in here, a tile into the next item: its
       // partials have drained, and the fence and the atomic's round trip cost one thread of
       // one group a microsecond in mid-stream instead of stalling an item boundary. The wait
       // (long satisfied) is what orders every worker warp's partial stores before this
       // thread's release fence and atomic.
-      if (wg == 0 && t == 0 && pend_k > 0 && seen < 0) {
-        mbar_wait(bars.stored(), pend_phase, abort_flag, status, 29, wprof);
-        __threadfence();
-        seen = atomicAdd(P.a.unit_counters + pend_unit, 1);
-      }
+      if (count_due) count_in();
     }
     it0 += nt;
-    FQ_ITEM_STAMP(24);
     if (pending) accumulate();
-    FQ_ITEM_STAMP(27);
 
     // ---- item epilogue. First, the count-in of the previous split piece (see step 1 below)
-    if (wg == 0 && t == 0 && pend_k > 0 && seen < 0) {   // group 0 had no tile in this item
-      mbar_wait(bars.stored(), pend_phase, abort_flag, status, 29, wprof);
-      __threadfence();
-      seen = atomicAdd(P.a.unit_counters + pend_unit, 1);
-    }
+    if (count_due) count_in();   // group 0 had no tile in this item
     // group sums, then the groups' states through shared memory
     float* rs = red_sum + (wg * 4 + wq) * 16;
 #pragma unroll
@@ -656,11 +506,14 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       for (int h = 0; h < GP; ++h) xo[h * TILE + t] = oacc[h];   // head-major: no bank conflicts
       if (t == 0) {
 #pragma unroll
-        for (int h = 0; h < GP; ++h) { xmeta[h] = m[h]; xmeta[8 + h] = l[h]; xmeta[16 + h] = c[h]; }
+        for (int h = 0; h < GP; ++h) {
+          xmeta[h] = (unset >> h) & 1u ? -INFINITY : m[h];
+          xmeta[8 + h] = l[h];
+          xmeta[16 + h] = c[h];
+        }
       }
     }
     named_barrier(1 + G, 128 * G);
-    FQ_ITEM_STAMP(30);
     // The groups' states are merged in fixed order (group 0, then 1, 2, 3), each group taking a
     // share of the heads; the loop over the groups is unrolled so that its loads go out together.
     // (The results go to global memory only after the barrier below: a barrier that follows
@@ -693,7 +546,6 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       }
       rM[i] = M; rL[i] = L; rO[i] = O;
     }
-    FQ_ITEM_STAMP(28);
     // ---- in-kernel merge, step 1. A split piece is counted in (release fence + one atomic on
     // its unit's counter) not here but a tile into the NEXT item (above), or after the last
     // item. Whoever finds the count complete makes the CTA merge that unit after the barrier
@@ -714,10 +566,9 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         pend_phase = static_cast<uint32_t>(ik & 1);
       }
     }
-    FQ_ITEM_STAMP(31);
+    if (warp == 0) count_due = w.slot >= 0 && P.a.unit_counters != nullptr;
     // the exchange buffers are reused by the next item
     named_barrier(1 + G, 128 * G);
-    FQ_ITEM_STAMP(25);
     // ---- in-kernel merge, step 2: every group takes its share of the unit's heads (the words
     // are next written after the next item's first all-group barrier, which this read precedes)
     if (w.slot != -2) {
@@ -750,7 +601,6 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
     if (lane == 0) mbar_arrive(bars.stored());
     if (merge_info[0] > 0)
       merge_unit(merge_info[0], merge_info[1], merge_info[2], merge_info[3], wg, G);
-    FQ_ITEM_STAMP(26);
   }
   // The last split piece of this CTA is counted in here; if that completes its unit, the CTA
   // merges it (every group its share of the heads, as above).
@@ -760,7 +610,7 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       int km = 0;
       if (pend_k > 0) {
         if (seen < 0) {
-          mbar_wait(bars.stored(), pend_phase, abort_flag, status, 29, wprof);
+          mbar_wait(bars.stored(), pend_phase, abort_flag, status);
           __threadfence();
           seen = atomicAdd(P.a.unit_counters + pend_unit, 1);
         }
@@ -780,30 +630,27 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
 }  // namespace
 
 template <int BITS, int D, int GP, int KG, bool MQ>
-__global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D)) decode_kernel(const DecodeParams P) {
+__global__ void __launch_bounds__(decode_threads(BITS, D), 1)
+decode_kernel(const __grid_constant__ DecodeParams P) {
   // KG: 1 whole-head K with f32 records, 3 the same with bf16 pairs, 2 two 64-channel K groups
   static_assert(KG == 1 || KG == 3 || (KG == 2 && D == 128),
                 "K groups of 64 channels at head_dim 128");
   static_assert(D == 64 || D == 128, "this build tiles head_dim 64 and 128");
   using SP = SmemPlan<BITS, D>;
   using TP = TmemPlan<BITS, D>;
-  constexpr int G = SP::G;
+  constexpr int G = SP::G, NS = SP::NS;
   constexpr int W_PRODUCER = 4 * G, W_S = W_PRODUCER + 1, W_PV = W_PRODUCER + 2,
                 W_PRODUCER2 = W_PRODUCER + 3;
   static_assert(decode_threads(BITS, D) == 32 * (W_PRODUCER2 + 1), "warp roles and block size disagree");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem = smem_raw + (smem0 - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int NS = P.ring_stages;
-  Bars<G> bars{smem0 + SP::BAR_OFF, NS};
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const Bars<G, NS> bars{smem0 + SP::BAR_OFF};
+  static_assert(8 * Bars<G, NS>::WORDS <= 1016, "barrier words");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SP::BAR_OFF + 1024);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SP::BAR_OFF + 1016);
   int* status = P.a.status;
-#ifdef FQ_WAIT_PROFILE
-  const long long kernel_t0 = clock64();
-  if (threadIdx.x < WAIT_SITES) const_cast<int*>(abort_flag)[4 + threadIdx.x] = 0;
-#endif
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -813,10 +660,9 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
       mbar_init(bars.ring_empty(s), 4);  // the four warps of the group that took the tile
     }
     for (int g = 0; g < G; ++g) {
-      mbar_init(bars.k_ready(g), 4);
       mbar_init(bars.s_done(g), 1);
-      mbar_init(bars.pv_ready(g), 4);
       mbar_init(bars.pv_done(g), 1);
+      mbar_init(bars.pv_ready(g), 4);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bars.q_full(s), 1);
@@ -829,7 +675,7 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
 
   // Everything above touched only this CTA's shared and tensor memory. Under a programmatic
   // launch it may have run while the launch before this one in the stream was still finishing:
@@ -838,7 +684,7 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  const ItemRange items = item_range(P);
+  const ItemRange items = uniform_range(item_range(P));
   // The CTA's first items, decoded by one thread each: their dependent loads (row, length, table
   // offset) go out side by side, once, instead of in every role at every item boundary.
   WorkItem* const item_cache = reinterpret_cast<WorkItem*>(smem + SP::ITEM_OFF);
@@ -854,10 +700,6 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
   }
   __syncthreads();
   const uint32_t ring0 = smem0 + SP::RING_OFF;
-  int wprof[WAIT_SITES] = {};   // used by the diagnostic build only
-#ifdef FQ_WAIT_PROFILE
-  if (threadIdx.x == 0) wprof[22] = static_cast<int>(clock64() - kernel_t0);   // set-up
-#endif
 
   if (warp == W_PRODUCER || warp == W_PRODUCER2) {
     // ------------------------------------------------------------------ producers
@@ -870,10 +712,16 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
     // B operand; it runs a ring's depth ahead of the MMAs, which hides the load.
     const int pi = warp == W_PRODUCER ? 0 : 1;
     const uint64_t stream_policy = l2_evict_first_policy();
+    // (the stage count is even: a producer's own tiles are two stages apart)
+    uint32_t stage = ring0 + pi * SP::STAGE, full = bars.ring_full(pi), empty_ph = 1;
+    // code chunks go to their swizzled place in the row (SmemPlan::row_swizzle); a lane's
+    // 16 bytes are chunk lane % CHUNKS of row lane / CHUNKS (+ a multiple of 8 rows)
+    const uint32_t code_lane = 16u * ((lane & ~(SP::CHUNKS - 1)) |
+                                      ((lane & (SP::CHUNKS - 1)) ^ SP::row_swizzle(lane / SP::CHUNKS)));
+    const uint64_t lane16 = 16u * lane;
     int it = 0, qi = 0;
-    RingPos rp;
     for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
-      const WorkItem w = item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi);
+      const WorkItem w = uniform_item(item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi));
       if (w.t1 <= w.t0) continue;
       constexpr int PPT = SP::PPT;   // pages per tile
       const int npages = (w.len + PAGE - 1) / PAGE;
@@ -895,7 +743,7 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
       int cur = fetch(PPT * w.t0);
       if (pi == 0) {
         const int qb = qi & 1;
-        mbar_wait(bars.q_empty(qb), ((qi >> 1) & 1) ^ 1, abort_flag, status, 7, wprof);
+        mbar_wait(bars.q_empty(qb), ((qi >> 1) & 1) ^ 1, abort_flag, status);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int chunk = lane + 32 * j;      // 16 rows of eight 16-byte chunks
@@ -905,9 +753,11 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
           // the K row (bytes 0-63) and rows 8-15 the same heads against the second's (64-127).
           // With two K groups of 64 channels (one token per lane) the same split of the rows
           // yields each group's partial product in its own S column.
-          constexpr bool SPLIT = SP::PAIR || KG == 2;
-          const int hl = w.ht * 8 + (SPLIT ? (r & 7) : r);  // head inside the KV head's group
-          const bool live = (SPLIT || r < 8) && hl < P.heads_per_kv;
+          // INT2 with whole-head K: rows 0-7 carry the heads against the even operand words, rows
+          // 8-15 the same heads against the odd ones, which hold 4 * code (expand_words_v).
+          constexpr bool SPLIT = SP::PAIR || KG == 2, ODD = odd_columns(BITS, D, KG);
+          const int hl = w.ht * 8 + (r & 7);        // head inside the KV head's group
+          const bool live = (SPLIT || ODD || r < 8) && hl < P.heads_per_kv;
           const long long qrow = live ? caller_row<MQ>(P, w.b, w.kvh, hl) : 0;
           const bool mine = SPLIT ? ((r < 8) == (cc < 4)) : 16 * cc < D;
           const int src = SP::PAIR ? (cc & 3) : cc;
@@ -928,6 +778,8 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
               v.y = __byte_perm(in.z, in.w, 0x6420);
               v.z = __byte_perm(in.x, in.y, 0x7531);
               v.w = __byte_perm(in.z, in.w, 0x7531);
+              if (ODD && r < 8) v.y = v.w = 0u;
+              if (ODD && r >= 8) v.x = v.z = 0u;
             } else {
               v = in;
             }
@@ -949,7 +801,7 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
               }
               float* hc = reinterpret_cast<float*>(smem + SP::HEADC_OFF) + qb * 24;
               if (r < 8) {
-                hc[r] = scale;
+                hc[r] = scale * 512.f;   // (a code byte is code * 2^-9)
                 hc[8 + r] = scale * qsum;
               } else {
                 hc[16 + (r - 8)] = scale * qsum;
@@ -962,37 +814,31 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
         if (lane == 0) mbar_arrive(bars.q_full(qb));
       }
       ++qi;
+      // this producer's tiles of the item: every other one
+      int k = (it ^ pi) & 1;
+      it += w.t1 - w.t0;
       for (int base = PPT * w.t0; base < PPT * w.t1; base += 32) {
         const int nxt = base + 32 < PPT * w.t1 ? fetch(base + 32) : -1;
-        for (int k = 0; k < 32 / PPT && base + PPT * k < PPT * w.t1; ++k, ++it) {
-          const int s = rp.s;
-          const uint32_t eph = rp.ph ^ 1u;
-          rp.next(NS);
-          if ((it & 1) != pi) continue;
-          int ids[PPT];
-#pragma unroll
-          for (int j = 0; j < PPT; ++j) ids[j] = __shfl_sync(0xFFFFFFFFu, cur, PPT * k + j);
-          mbar_wait(bars.ring_empty(s), eph, abort_flag, status, 0, wprof);
-          const uint32_t full = bars.ring_full(s);
-          // code chunks go to their swizzled place in the row (SmemPlan::row_swizzle); a lane's
-          // 16 bytes are chunk lane % CHUNKS of row lane / CHUNKS (+ a multiple of 8 rows)
-          const int code_lane = (lane & ~(SP::CHUNKS - 1)) |
-                                ((lane & (SP::CHUNKS - 1)) ^ SP::row_swizzle(lane / SP::CHUNKS));
-          const uint32_t dst = ring0 + s * SP::STAGE + 16 * code_lane;
-          const uint32_t dst_rec = ring0 + s * SP::STAGE + 16 * lane;
+        const int stop = min(32, PPT * w.t1 - base);
+#pragma unroll 1
+        for (int pg = PPT * k; pg < stop; pg += 2 * PPT) {
+          mbar_wait_warp(full + 8 * NS, empty_ph, abort_flag, status);
 #pragma unroll
           for (int j = 0; j < PPT; ++j) {
-            const int id = ids[j];
-            if (id < 0 || (FQ_STUB_ROLES & 8)) continue;
-            const long long blk = static_cast<long long>(id) * P.p.num_kv_heads + w.kvh;
-            const uint8_t* ks = P.p.k_codes + blk * SP::CODE_PAGE + 16 * lane;
-            const uint8_t* vs = P.p.v_codes + blk * SP::CODE_PAGE + 16 * lane;
+            const int id = __shfl_sync(0xFFFFFFFFu, cur, pg + j);
+            if (id < 0) continue;
+            // (blocks are numbered below 2^32: one is at least 2.5 KB)
+            const uint32_t blk = static_cast<uint32_t>(id) * P.p.num_kv_heads + w.kvh;
+            const uint64_t off = static_cast<uint64_t>(blk) * SP::CODE_PAGE + lane16;
+            const uint8_t* ks = P.p.k_codes + off;
+            const uint8_t* vs = P.p.v_codes + off;
             // records: 16 B per token in an f32 pool, 8 B in a bf16 pool (same slot in the ring)
             // (with two K groups: 8 B of K pairs per token, then 4 B of V pairs per token)
             constexpr int scale_page =
                 KG == 2 ? 12 * PAGE : (KG == 3 ? SP::SCALE_PAGE / 2 : SP::SCALE_PAGE);
-            const uint8_t* ss = static_cast<const uint8_t*>(P.p.scales) + blk * scale_page +
-                                16 * lane;
+            const uint8_t* ss = static_cast<const uint8_t*>(P.p.scales) +
+                                (static_cast<uint64_t>(blk) * scale_page + lane16);
+            const uint32_t dst = stage + code_lane, dst_rec = stage + 16 * lane;
 #pragma unroll
             for (int c = 0; c < SP::CODE_PAGE; c += 512)
               cp_async16_stream(dst + SP::K_OFF + j * SP::CODE_PAGE + c, ks + c, stream_policy);
@@ -1001,96 +847,78 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
               cp_async16_stream(dst + SP::V_OFF + j * SP::CODE_PAGE + c, vs + c, stream_policy);
 #pragma unroll
             for (int c = 0; c < SP::SCALE_PAGE; c += 512)
-              if (c + 16 * lane < scale_page)
+              if (c + 512 <= scale_page || c + 16 * lane < scale_page)
                 cp_async16_stream(dst_rec + SP::S_OFF + j * SP::SCALE_PAGE + c, ss + c,
                                   stream_policy);
           }
           cp_async_arrive(full);
+          stage += 2 * SP::STAGE;
+          full += 16;
+          if (full >= bars.ring_full(NS)) {
+            stage -= NS * SP::STAGE;
+            full -= 8 * NS;
+            empty_ph ^= 1u;
+          }
         }
         cur = nxt;
       }
     }
-    // drain: every copy this warp issued has landed once its stage reports full
-    for (int back = 0; back < NS && back < it; ++back) {
-      if (--rp.s < 0) { rp.s = NS - 1; rp.ph ^= 1u; }
-      mbar_wait_drain(bars.ring_full(rp.s), rp.ph, P.wait_budget / 16);
-    }
+    // every copy this warp issued has landed before the CTA's shared memory is released
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == W_S) {
     // ------------------------------------------------------------------ S issuer
-    // One thread issues S = C_K . Q^T for every tile, in tile order. The loop is kept to a few
-    // dozen scalar instructions per tile: descriptor high words, the instruction descriptor and
-    // the accumulate flags are immediates, and the group index is a counter.
-    if (lane == 0) {
-      constexpr uint32_t IDESC_S = make_idesc_e4m3(128, 16, 0, 0);
-      constexpr uint32_t Q_HI = smem_desc_hi(1024, 2);
-      int qi = 0, g = 0;   // tiles go to the groups in turn
-      uint32_t gph = 0;    // phase of the groups' barriers: flips once per round of G tiles
-      for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
-        const WorkItem w = item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi);
-        if (w.t1 <= w.t0) continue;
-        const int qb = qi & 1;
-        mbar_wait(bars.q_full(qb), (qi >> 1) & 1, abort_flag, status, 1, wprof);
-        const uint32_t q_lo = smem_desc_lo(smem0 + SP::Q_OFF + qb * SP::Q_BYTES, 16);
-        for (int t = w.t0; t < w.t1; ++t) {
-          mbar_wait(bars.k_ready(g), gph, abort_flag, status, 2, wprof);
-          tc_fence_after();
-          // (with a 128-byte row per token, a chain and a 16-column S buffer per token)
-#pragma unroll
-          for (int u = 0; u < (SP::TWO ? 2 : 1); ++u) {
-            const uint32_t sd = tmem + TP::S + g * TP::S_COLS + 16 * u;
-            const uint32_t ka = tmem + TP::KOP + g * TP::KOP_COLS + (D / 4) * u;
-            umma_ts_c<Q_HI, IDESC_S, false>(sd, ka, q_lo);
-#pragma unroll
-            for (int k = 1; k < ((FQ_STUB_ROLES & 16) ? 1 : (SP::PAIR ? 2 : 1) * D / 32); ++k)
-              umma_ts_c<Q_HI, IDESC_S, true>(sd, ka + 8 * k, q_lo + 2 * k);
-          }
-          tc_commit(bars.s_done(g));
-          if (t == w.t1 - 1) tc_commit(bars.q_empty(qb));
-          if (++g == G) { g = 0; gph ^= 1u; }
-        }
-        ++qi;
+    // The whole warp walks the tiles; one elected lane issues S = C_K . Q^T. The group index is
+    // a counter, descriptor high words, the instruction descriptor and the accumulate flags are
+    // immediates.
+    constexpr uint32_t IDESC_S = make_idesc_e4m3(128, 16, 0, 0);
+    constexpr uint32_t Q_HI = smem_desc_hi(1024, 2);
+    int qi = 0, g = 0;   // tiles go to the groups in turn
+    for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
+      const WorkItem w = uniform_item(item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi));
+      if (w.t1 <= w.t0) continue;
+      const int qb = qi & 1;
+      mbar_wait_warp(bars.q_full(qb), (qi >> 1) & 1, abort_flag, status);
+      const uint32_t q_lo = smem_desc_lo(smem0 + SP::Q_OFF + qb * SP::Q_BYTES, 16);
+#pragma unroll 1
+      for (int t = w.t0; t < w.t1; ++t) {
+        named_barrier(K_READY<G> + g, 160);
+        tc_fence_after();
+        umma_ts_chain4<Q_HI, IDESC_S>(tmem + TP::S + g * TP::S_COLS, tmem + TP::KOP + g * TP::KOP_COLS,
+                                      q_lo, bars.s_done(g));
+        if (++g == G) g = 0;
       }
+      tc_commit_elect(bars.q_empty(qb));   // after the item's last chain
+      ++qi;
     }
-    __syncwarp();
   } else if (warp == W_PV) {
     // ------------------------------------------------------------------ PV issuer
-    if (lane == 0) {
-      constexpr uint32_t IDESC_PV = make_idesc_e4m3(128, 16, 1, 1);
-      constexpr uint32_t V_HI = smem_desc_hi(1024, 2), P_HI = smem_desc_hi(128, 0);
-      const uint32_t v_lo0 = smem_desc_lo(smem0 + SP::VOP_OFF, 16);
-      const uint32_t p_lo0 = smem_desc_lo(smem0 + SP::P_OFF, 128);
-      int g = 0;
-      uint32_t gph = 0;
-      for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
-        const WorkItem w = item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi);
-        for (int t = w.t0; t < w.t1; ++t) {
-          mbar_wait(bars.pv_ready(g), gph, abort_flag, status, 4, wprof);
-          tc_fence_after();
-          const uint32_t v_lo = v_lo0 + g * (SP::VOP_STAGE >> 4);
-          const uint32_t p_lo = p_lo0 + g * (SP::P_BYTES >> 4);
-          const uint32_t od = tmem + TP::O + g * TP::O_COLS;
-          // one accumulator per token of a lane: the same V rows against that token's P plane
-#pragma unroll
-          for (int u = 0; u < (SP::PAIR ? 2 : 1); ++u) {
-            const uint32_t pu = p_lo + u * (TILE * 16 >> 4);
-            umma_ss_c<V_HI, P_HI, IDESC_PV, false>(od + 16 * u, v_lo, pu);
-#pragma unroll
-            for (int k = 1; k < ((FQ_STUB_ROLES & 32) ? 1 : (SP::TWO ? 2 : 1) * TILE / 32); ++k)
-              umma_ss_c<V_HI, P_HI, IDESC_PV, true>(od + 16 * u, v_lo + k * (32 * SP::ROW >> 4),
-                                                    pu + k * (32 * 16 >> 4));
-          }
-          tc_commit(bars.pv_done(g));
-          if (++g == G) { g = 0; gph ^= 1u; }
-        }
+    constexpr uint32_t IDESC_PV = make_idesc_e4m3(128, 16, 1, 1);
+    constexpr uint32_t V_HI = smem_desc_hi(1024, 2), P_HI = smem_desc_hi(128, 0);
+    const uint32_t v_lo0 = smem_desc_lo(smem0 + SP::VOP_OFF, 16);
+    const uint32_t p_lo0 = smem_desc_lo(smem0 + SP::P_OFF, 128);
+    int g = 0;
+    uint32_t gph = 0;    // phase of the groups' barriers: flips once per round of G tiles
+    for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
+      const WorkItem w = uniform_item(item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi));
+#pragma unroll 1
+      for (int t = w.t0; t < w.t1; ++t) {
+        mbar_wait_warp(bars.pv_ready(g), gph, abort_flag, status);
+        tc_fence_after();
+        const uint32_t v_lo = v_lo0 + g * (SP::VOP_STAGE >> 4);
+        const uint32_t p_lo = p_lo0 + g * (SP::P_BYTES >> 4);
+        const uint32_t od = tmem + TP::O + g * TP::O_COLS;
+        // one accumulator per token of a lane: the same V rows against that token's P plane
+        umma_ss_chain4<V_HI, P_HI, IDESC_PV, (32 * SP::ROW >> 4), (32 * 16 >> 4)>(od, v_lo, p_lo);
+        if constexpr (SP::PAIR)
+          umma_ss_chain4<V_HI, P_HI, IDESC_PV, (32 * SP::ROW >> 4), (32 * 16 >> 4)>(
+              od + 16, v_lo, p_lo + (TILE * 16 >> 4));
+        tc_commit_elect(bars.pv_done(g));
+        if (++g == G) { g = 0; gph ^= 1u; }
       }
     }
-    __syncwarp();
   } else {
     // ------------------------------------------------------------------ workers
-    worker_role<BITS, D, GP, KG, MQ>(P, smem, smem0, tmem, bars, abort_flag, items, wprof);
-#ifdef FQ_WAIT_PROFILE
-    if (threadIdx.x == 0) wprof[21] = static_cast<int>(clock64() - kernel_t0);   // workers done
-#endif
+    worker_role<BITS, D, GP, KG, MQ>(P, smem, smem0, tmem, bars, abort_flag, items);
   }
 
   tc_fence_before();
@@ -1099,19 +927,6 @@ __global__ void __launch_bounds__(decode_threads(BITS, D), ctas_per_sm(BITS, D))
     tc_fence_after();
     tmem_dealloc(tmem, TP::ALLOC);
   }
-#ifdef FQ_WAIT_PROFILE
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < WAIT_SITES; ++i)
-      if (wprof[i]) atomicAdd(const_cast<int*>(abort_flag) + 4 + i, wprof[i] >> 4);
-  }
-  __syncthreads();
-  if (g_wait_profile != nullptr && threadIdx.x < WAIT_SITES) {
-    int v = const_cast<int*>(abort_flag)[4 + threadIdx.x];
-    if (threadIdx.x == 23) v = static_cast<int>((clock64() - kernel_t0) >> 4);
-    g_wait_profile[blockIdx.x * WAIT_SITES + threadIdx.x] = v;
-  }
-#endif
 }
 
 // Tensor-core self test (see foscar_b200.h): one tile of both contractions on given operands.
@@ -1241,29 +1056,16 @@ static int device_sm_count() {
 template <int BITS, int D, int GP, int KG = 1, bool MQ = false>
 static int launch_decode(DecodeParams& P, cudaStream_t stream) {
   using SP = SmemPlan<BITS, D>;
-  constexpr int THREADS = decode_threads(BITS, D);
-  int stages = SP::max_ring_stages();
-  if (stages > 20) stages = 20;
-  if (const char* env = getenv("FOSCAR_B200_RING_STAGES")) {   // tuning knob for experiments
-    const int want = atoi(env);
-    if (want >= SP::G && want < stages) stages = want;
-  }
-  // An even ring: the two producers take alternate tiles, so with an even stage count a stage
-  // always belongs to the same producer, which then sees every release of it. With an odd count
-  // a producer meets a stage every second lap only and waits on a phase parity that an older,
-  // still outstanding release also satisfies (a 5-stage ring hung on exactly that).
-  stages &= ~1;
-  if (stages < SP::G) return FQ_ERR_UNSUPPORTED;  // a group steps the ring by one lap at most
-  P.ring_stages = stages;
+  constexpr int THREADS = decode_threads(BITS, D), LIMIT = SMEM_LIMIT;
+  P.ring_stages = SP::NS;
   P.tile_tokens = SP::TT;
   P.wait_budget = P.a.wait_budget_cycles > 0 ? P.a.wait_budget_cycles : WAIT_BUDGET_CYCLES;
   // Shared memory the ring leaves over holds more decoded work items (32 bytes each), up to
   // one per thread of the CTA's start-up pass.
-  constexpr int LIMIT = smem_limit(BITS, D);
-  const int spare = LIMIT - 1024 - SP::RING_OFF - stages * SP::STAGE;
-  const int more = std::max(0, std::min(spare / 32, THREADS - SP::ITEM_SLOTS));
+  constexpr int spare = LIMIT - 1024 - SP::RING_OFF - SP::NS * SP::STAGE;
+  constexpr int more = std::max(0, std::min(spare / 32, THREADS - SP::ITEM_SLOTS));
   P.item_slots = SP::ITEM_SLOTS + more;
-  const int smem = SP::RING_OFF + stages * SP::STAGE + more * 32 + 1024;
+  constexpr int smem = SP::RING_OFF + SP::NS * SP::STAGE + more * 32 + 1024;
   static bool configured[64] = {};  // per (BITS, D, GP) instantiation and device
   auto kernel = decode_kernel<BITS, D, GP, KG, MQ>;
   int dev = 0;
@@ -1274,7 +1076,7 @@ static int launch_decode(DecodeParams& P, cudaStream_t stream) {
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev >= 0 && dev < 64) configured[dev] = true;
   }
-  int ctas = P.a.max_ctas > 0 ? P.a.max_ctas : device_sm_count() * ctas_per_sm(BITS, D);
+  int ctas = P.a.max_ctas > 0 ? P.a.max_ctas : device_sm_count();
   int grid = P.a.worklist ? ctas : std::min(ctas, P.num_items);
   if (grid < 1) grid = 1;
   if (P.a.flags & 1) {
@@ -1302,7 +1104,7 @@ using namespace fq;
 extern "C" int fq_ctas_per_sm(int32_t bits, int32_t head_dim) {
   if ((bits != 2 && bits != 4) || (head_dim != 64 && head_dim != 128 && head_dim != 256))
     return FQ_ERR_UNSUPPORTED;
-  return head_dim == 256 ? 1 : ctas_per_sm(bits, head_dim);
+  return 1;
 }
 
 extern "C" int fq_tile_tokens(int32_t bits, int32_t head_dim) {
@@ -1440,11 +1242,6 @@ extern "C" int fq_decode_split_static(const fq_pools* pools, const fq_decode_arg
                   a.out_dtype, a.lse, stream);
 }
 
-#ifdef FQ_WAIT_PROFILE
-extern "C" int fq_debug_set_wait_profile(void* buffer) {
-  return static_cast<int>(cudaMemcpyToSymbol(fq::g_wait_profile, &buffer, sizeof(buffer)));
-}
-#endif
 
 extern "C" int fq_umma_selftest(int32_t mode, const uint8_t* k_bytes, const uint8_t* q_bytes,
                                 const uint8_t* v_bytes, const uint8_t* p_bytes, float* s_out,

@@ -6,53 +6,18 @@
 namespace fq {
 
 constexpr int TILE = 128;            // MMA rows: tensor-memory lanes, threads of a worker group
-// Tokens per sequence tile. head_dim 128: one token per lane (two pages). head_dim 64: two tokens
-// per lane, t and 128 + t of the tile (four pages): their 64-byte operand rows sit side by side
-// in one 128-byte row, so a tile of 256 tokens costs what a 128-token tile of head_dim 128 costs.
-// INT2 at head_dim 128 can be built the same way (-DFQ_INT2_TWO_TOKENS=1): two tokens per lane,
-// each with a 128-byte operand row and a score chain of its own, in three worker groups instead
-// of four (the V operand stage of 256 tokens is 32 KB a group), so that the per-tile waits,
-// barriers, tensor-memory round trips and the O accumulation are paid once per 256 tokens. It
-// passes the same tests and was measured no faster (long contexts +1 %, mixed batches +5 to
-// +14 %), so the build with one token per lane is the default.
-#ifndef FQ_INT2_TWO_TOKENS
-#define FQ_INT2_TWO_TOKENS 0
-#endif
-__host__ __device__ constexpr bool two_token_build(int bits, int head_dim) {
-  return FQ_INT2_TWO_TOKENS != 0 && bits == 2 && head_dim == 128;
-}
-__host__ __device__ constexpr int tile_tokens(int bits, int head_dim) {
-  return head_dim == 64 || two_token_build(bits, head_dim) ? 256 : 128;
-}
+// Tokens per sequence tile. head_dim 128 and 256: one token per lane (two pages). head_dim 64: two
+// tokens per lane, t and 128 + t of the tile (four pages): their 64-byte operand rows sit side by
+// side in one 128-byte row, so a tile of 256 tokens costs what a 128-token tile of head_dim 128
+// costs.
+__host__ __device__ constexpr int tile_tokens(int, int head_dim) { return head_dim == 64 ? 256 : 128; }
 constexpr int WORK_WORDS = 8;        // int32 words per explicit work-list row
-#ifndef FQ_WORKER_GROUPS
-#define FQ_WORKER_GROUPS 4
-#endif
-constexpr int WORKER_GROUPS = FQ_WORKER_GROUPS;  // 128-thread groups, tile i -> group i % G
-// Two CTAs of two worker groups each per SM instead of one CTA of four (-DFQ_INT2_TWO_CTAS=1,
-// the INT2 builds): the CTAs' item epilogues and prologues overlap each other's tiles; each gets
-// half the shared memory (the INT4 rings would be too shallow). Measured 16 to 31 % slower than
-// one CTA of four groups on every workload tried, so it is off.
-#ifndef FQ_INT2_TWO_CTAS
-#define FQ_INT2_TWO_CTAS 0
-#endif
-__host__ __device__ constexpr int ctas_per_sm(int bits, int head_dim) {
-  return FQ_INT2_TWO_CTAS != 0 && bits == 2 && head_dim <= 128 && !two_token_build(bits, head_dim)
-             ? 2 : 1;
-}
-__host__ __device__ constexpr int worker_groups(int bits, int head_dim) {
-  return two_token_build(bits, head_dim) ? 3 : (ctas_per_sm(bits, head_dim) == 2 ? 2 : WORKER_GROUPS);
-}
-// + 2 producers + 2 MMA issuers
+// Worker groups of 128 threads, tile i -> group i % G; with them two producers and two MMA issuers.
+__host__ __device__ constexpr int worker_groups(int bits, int head_dim) { return 4; }
 __host__ __device__ constexpr int decode_threads(int bits, int head_dim) {
   return 32 * (4 * worker_groups(bits, head_dim) + 4);
 }
 constexpr int SMEM_LIMIT = 232448;   // 227 KiB opt-in limit per CTA on sm_100
-// (two CTAs per SM: half of the SM's 228 KiB less the KiB the system keeps per CTA)
-__host__ __device__ constexpr int smem_limit(int bits, int head_dim) {
-  return ctas_per_sm(bits, head_dim) == 2 ? 115712 : SMEM_LIMIT;
-}
-
 struct DecodeParams {
   fq_pools p;
   fq_decode_args a;  // num_qo_heads here counts a unit's columns: q_len x the caller's heads
@@ -129,9 +94,8 @@ struct SmemPlan {
     return CHUNKS == 4 ? (row >> 1) & 3 : (CHUNKS == 2 ? (row >> 2) & 1 : 0);
   }
   static constexpr int TT = tile_tokens(BITS, D);      // tokens per tile
-  static constexpr int G = worker_groups(BITS, D);     // worker groups of this build
+  static constexpr int G = worker_groups(BITS, D);
   static constexpr bool PAIR = D == 64;                // two tokens per lane, rows side by side
-  static constexpr bool TWO = TT == 2 * TILE && !PAIR; // two tokens per lane, a row each
   static constexpr int PPT = TT / PAGE;                // pages per tile
   static constexpr int K_OFF = 0;                      // a ring stage: K pages, V pages, records
   static constexpr int V_OFF = PPT * CODE_PAGE;
@@ -140,7 +104,7 @@ struct SmemPlan {
   // Operand rows keep a 128-byte pitch (the swizzle atom) whatever D <= 128: head_dim 64 uses
   // the first half of each row.
   static constexpr int ROW = 128;
-  static constexpr int VOP_STAGE = (TWO ? 2 : 1) * TILE * ROW;   // expanded V operand, one tile
+  static constexpr int VOP_STAGE = TILE * ROW;   // expanded V operand, one tile
   static constexpr int Q_BYTES = 16 * ROW;             // 16 MMA rows
   static constexpr int P_BYTES = TT * 16;              // 16 bytes (8 hi + 8 lo) per token, a
                                                        // plane of 128 rows per token of a lane
@@ -168,9 +132,14 @@ struct SmemPlan {
   static constexpr int ITEM_OFF = BAR_OFF + 1280;
   static constexpr int ITEM_SLOTS = (BAR_BYTES - 1280) / 32;
   static constexpr int RING_OFF = (BAR_OFF + BAR_BYTES + 1023) / 1024 * 1024;
-  static constexpr int max_ring_stages() {
-    return (smem_limit(BITS, D) - 1024 /*alignment slack*/ - RING_OFF) / STAGE;
+  // Ring stages: even, so that a stage always belongs to the same one of the two producers, which
+  // then sees every release of it.
+  static constexpr int stages() {
+    const int s = (SMEM_LIMIT - 1024 /*alignment slack*/ - RING_OFF) / STAGE;
+    return (s < 20 ? s : 20) & ~1;
   }
+  static constexpr int NS = stages();
+  static_assert(NS >= G, "a group steps the ring by one lap at most");
 };
 
 // The items a launch runs, decoded the same way by every role of every CTA.
@@ -231,6 +200,18 @@ struct ItemRange {
   int begin, end, step;
 };
 
+// A value that is the same in every lane, told to the compiler: it may then live in a uniform
+// register, where tensor-memory, barrier and descriptor operands have to be.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, 0); }
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xFFFFFFFFu, x, 0); }
+__device__ __forceinline__ WorkItem uniform_item(const WorkItem& w) {
+  return WorkItem{uniform(w.b), uniform(w.kvh), uniform(w.ht), uniform(w.t0),
+                  uniform(w.t1), uniform(w.slot), uniform(w.len), uniform(w.table_off)};
+}
+__device__ __forceinline__ ItemRange uniform_range(const ItemRange& r) {
+  return ItemRange{uniform(r.begin), uniform(r.end), uniform(r.step)};
+}
+
 // The CTA's k-th item (list index wi). The first items of a CTA (ITEM_SLOTS, plus as many as fit
 // in the shared memory the ring leaves over: DecodeParams::item_slots in all) are decoded once,
 // in parallel, when the CTA starts and kept in shared memory, so that no role pays the chain of
@@ -274,12 +255,40 @@ __device__ inline uint32_t f16x2_to_e4m3x2(__half2 x) {
   asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(r) : "r"(*reinterpret_cast<uint32_t*>(&x)));
   return r;
 }
+// Four f16 as two E4M3 planes: hi = e4m3(w), lo = e4m3(16 (w - hi)).
+__device__ __forceinline__ void split_e4m3x4(__half2 w0, __half2 w1, uint32_t& hi, uint32_t& lo) {
+  asm("{\n\t.reg .b16 a, b;\n\t.reg .b32 x, y, s;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f16x2 a, %2;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f16x2 b, %3;\n\t"
+      "mov.b32 %0, {a, b};\n\t"
+      "cvt.rn.f16x2.e4m3x2 x, a;\n\t"
+      "cvt.rn.f16x2.e4m3x2 y, b;\n\t"
+      "mov.b32 s, 0x4C004C00;\n\t"
+      "sub.f16x2 x, %2, x;\n\t"
+      "sub.f16x2 y, %3, y;\n\t"
+      "mul.f16x2 x, x, s;\n\t"
+      "mul.f16x2 y, y, s;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f16x2 a, x;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f16x2 b, y;\n\t"
+      "mov.b32 %1, {a, b};\n\t}"
+      : "=&r"(hi), "=r"(lo)
+      : "r"(*reinterpret_cast<const uint32_t*>(&w0)), "r"(*reinterpret_cast<const uint32_t*>(&w1)));
+}
 __device__ inline __half2 e4m3x2_to_f16x2(uint32_t v) {
   uint32_t r;
   asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"(static_cast<uint16_t>(v)));
   return *reinterpret_cast<__half2*>(&r);
 }
 
+// The same with the row given by its swizzled piece 0: piece v sits at `src` xor 16 v.
+template <int BITS, int D>
+__device__ __forceinline__ void load_code_row(uint32_t src, uint32_t (&w)[D * BITS / 32]) {
+#pragma unroll
+  for (int v = 0; v < D * BITS / 128; ++v)
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(w[4 * v]), "=r"(w[4 * v + 1]), "=r"(w[4 * v + 2]), "=r"(w[4 * v + 3])
+                 : "r"(src ^ (v << 4)));
+}
 // Load this thread's token row (RB bytes at `src`) as packed words.
 template <int BITS, int D>
 __device__ inline void load_row(uint32_t src, uint32_t (&w)[D * BITS / 32], int swz) {
