@@ -31,11 +31,11 @@ extern "C" int64_t fq_workspace_bytes(int32_t max_splits, int32_t batch, int32_t
   return 4ll * max_splits * batch * num_qo_heads * (head_dim + 2);
 }
 
-// Fixed cost of a piece in tile units (pipeline refill, the merge of the groups' states and the
-// output), as measured on B200 against the cost of streaming one tile (about 4.7 us against
-// 0.34 us per 128-token INT2 tile at head_dim 128).
+// Fixed cost of a piece in tile units (pipeline refill, the merge of the warps' or groups' states and
+// the output). Swept on B200 (6, 10, 14, 20, 28): at head_dim 128 six to fourteen are within 1 to 2 %; at head_dim 64, where a tile is half the bytes a token and an item ends in one warp's
+// merge, 256 requests of 64-131072 tokens took 652, 568, 521, 509 and 546 us; head_dim 256 as before.
 static long long piece_overhead(int bits, int head_dim) {
-  long long ovh = bits == 4 && head_dim == 128 ? 10 : 14;
+  long long ovh = head_dim == 64 ? 20 : (bits == 4 && head_dim == 128 ? 10 : 14);
   if (const char* env = getenv("FOSCAR_B200_PIECE_OVERHEAD")) {   // tuning knob for experiments
     const int v = atoi(env);
     if (v >= 0 && v <= 256) ovh = v;

@@ -1,4 +1,4 @@
-// Paged GQA decode attention over packed INT2/INT4 KV, sm_100a.
+// Paged GQA decode attention over packed INT2/INT4 KV at head_dim 128, sm_100a.
 //
 // What it computes follows the reference decode's semantics (src/foscar/wrapper.py:1153-1171;
 // fold algebra src/foscar/_sm100/int_fold_decode.py:5-22, 378-434): codes are never
@@ -37,21 +37,16 @@
 // and descriptor operands have to be in uniform registers. A tile took 1930 warp instructions with
 // lane-0 branches and run-time offsets and takes 1490; on one box 32 requests of 4K-32K tokens (INT2,
 // 32/8 heads) went from 107.8 to 97.4 us, 16 requests of 16K with two query tokens from 66.7 to
-// 55.7, the head_dim 64 build on 256 requests of 64-131072 tokens from 707 to 595. Three, five and
-// six groups measure the same or slower (the registers they cost), and so does one MMA in place of a
+// 55.7. Three, five and six groups measure the same or slower (the registers they cost), and so does one MMA in place of a
 // chain of four: what is left is the instructions' own latency at five warps a scheduler.
 // Every role walks the same list of work items, so the pipeline never drains inside an item.
 // Byte-expansion yields channels in a fixed permuted order; Q is loaded in that order and O is
 // stored through it, so no per-element fix-up exists anywhere.
 //
 // Variants of the same code (template parameters):
-//   head_dim 64   a tile is 256 tokens, two per lane (t and 128 + t): their K rows side by side
-//                 in the lane's 128-byte tensor-memory row, their V rows side by side in one
-//                 shared-memory row; query rows 0-7 act on bytes 0-63 and rows 8-15 on bytes
-//                 64-127, so one chain of S MMAs gives both tokens' scores (columns h, 8 + h);
-//                 the PV MMA runs once per token set into its own 16 accumulator columns.
-//   KG == 2       K quantized over two 64-channel groups (head_dim 128): the same split of the
-//                 query rows puts each group's partial score in its own column.
+//   KG == 2       K quantized over two 64-channel groups: query rows 0-7 carry the heads against
+//                 the first group's half of the row, rows 8-15 against the second's, which puts
+//                 each group's partial score in its own column.
 //   KG == 3       whole-head K with bf16 record pairs (8 bytes a token) instead of f32 (16).
 // Split units are merged inside this launch: a piece that wrote partials is counted in on its
 // unit's counter one tile into the CTA's next item (or after its last), once every worker warp
@@ -93,8 +88,7 @@ struct Bars {
 template <int G> constexpr int K_READY = 2 + G;
 
 // Tensor-memory column plan (f32 columns): per worker group one K operand stage (a 128-byte row
-// per lane; at head_dim 64 a lane holds two tokens), one S buffer of 16 columns and one O buffer
-// of 16 columns per token of a lane.
+// per lane), one S buffer and one O buffer of 16 columns.
 // INT2 with whole-head K at head_dim 128: the K rows are unpacked like the V rows, at five instead
 // of seven instructions a packed word (odd operand words hold 4 * code), and the idle half of the
 // sixteen query rows takes the odd words' products into score columns 8-15.
@@ -104,11 +98,10 @@ __host__ __device__ constexpr bool odd_columns(int bits, int head_dim, int kg) {
 
 template <int BITS, int D>
 struct TmemPlan {
-  static constexpr int G = worker_groups(BITS, D);
-  static constexpr bool PAIR = D == 64;
+  static constexpr int G = WORKER_GROUPS;
   static constexpr int KOP_COLS = 32;
   static constexpr int S_COLS = 16;
-  static constexpr int O_COLS = PAIR ? 32 : 16;
+  static constexpr int O_COLS = 16;
   static constexpr int KOP = 0;
   static constexpr int S = G * KOP_COLS;
   static constexpr int O = S + G * S_COLS;
@@ -119,19 +112,15 @@ struct TmemPlan {
 
 // The request's last tile with several query tokens per request: column h sees positions below
 // len - lag(h) only. Out of line, so that this rare path (and column_lag's division) costs the
-// tile loop nothing: the scores pass through local memory here and nowhere else. `pos0` is the
-// thread's first token position of the tile, `stride` the distance to its next one. Returns,
-// in `over`, the largest visible score.
-template <int NT, int GP>
-__device__ __noinline__ void mask_lagged_columns(const DecodeParams& P, int len, int ht, int pos0,
-                                                 int stride, float (&x)[NT][GP], float& over) {
+// tile loop nothing: the scores pass through local memory here and nowhere else. `pos` is the
+// thread's token position. Returns, in `over`, the largest visible score.
+template <int GP>
+__device__ __noinline__ void mask_lagged_columns(const DecodeParams& P, int len, int ht, int pos,
+                                                 float (&x)[GP], float& over) {
   float top = -INFINITY;
   for (int h = 0; h < GP; ++h) {
-    const int lim = len - column_lag(P, ht * 8 + h);
-    for (int u = 0; u < NT; ++u) {
-      if (pos0 + u * stride >= lim) x[u][h] = -INFINITY;
-      top = fmaxf(top, x[u][h]);
-    }
+    if (pos >= len - column_lag(P, ht * 8 + h)) x[h] = -INFINITY;
+    top = fmaxf(top, x[h]);
   }
   over = top;
 }
@@ -156,11 +145,8 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
   const uint32_t lane_base = static_cast<uint32_t>(32 * wq) << 16;
   const uint32_t k_dst = tmem + lane_base + TP::KOP + wg * TP::KOP_COLS;
   const uint32_t s_src = tmem + lane_base + TP::S + wg * TP::S_COLS;
-  constexpr int NT = SP::TT / TILE;   // tokens per lane
   constexpr bool ODD = odd_columns(BITS, D, KG);
-  // a lane's O columns: at two tokens per lane, rows 0-63 (warps 0, 1) hold the first token
-  // set's channels and take its P columns, rows 64-127 the second's
-  const uint32_t o_src = tmem + lane_base + TP::O + wg * TP::O_COLS + (SP::PAIR && wq >= 2 ? 16 : 0);
+  const uint32_t o_src = tmem + lane_base + TP::O + wg * TP::O_COLS;
   // (rows are 128 bytes at a 1024-byte aligned base: piece cc of the swizzled row is an xor away)
   const uint32_t v_row = (smem0 + SP::VOP_OFF + wg * SP::VOP_STAGE + t * SP::ROW) | ((t & 7) << 4);
   const uint32_t p_row = smem0 + SP::P_OFF + wg * SP::P_BYTES + t * 16;
@@ -199,8 +185,7 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
   const float o_mul = exp2f(static_cast<float>(9 - lp));
 
   auto merge_unit = [&](int k, int b, int kvh, int ht, int h0, int hstep) {
-    if (t < D)
-      merge_unit_partials<MQ, 1>(P, D, GP, channel_of_expanded_pos<BITS>(t), t == 0, k, b, kvh, ht, h0,
+    merge_unit_partials<MQ, 1>(P, D, GP, channel_of_expanded_pos<BITS>(t), t == 0, k, b, kvh, ht, h0,
                           hstep);
   };
   // the split piece this CTA has written but not yet counted in (thread 0 of group 0 only)
@@ -280,19 +265,9 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
 #pragma unroll 1
     for (; mine < it0 + nt; mine += G, pos0 += G * SP::TT) {
       mbar_wait_warp(full, ring_ph, abort_flag, status);
-      // ---- K row(s) -> tensor memory (the S MMA's A operand). The stage is free: this group
-      // read the S of its previous tile, so that tile's MMA, the stage's last reader, is
-      // complete. With two tokens per lane (head_dim 64) the second token's 64 bytes follow the
-      // first's in the lane's 128-byte row.
-      if constexpr (SP::PAIR) {
-#pragma unroll 1
-        for (int u = 0; u < 2; ++u) {
-          uint32_t wk[64 * BITS / 32], op[16];
-          load_code_row<BITS, 64>(stage + SP::K_OFF + u * TILE * SP::RB + code_row, wk);
-          expand_words<BITS, 64>(wk, op);
-          tmem_st16(k_dst + 16 * u, op);
-        }
-      } else {
+      // ---- K row -> tensor memory (the S MMA's A operand). The stage is free: this group read the
+      // S of its previous tile, so that tile's MMA, the stage's last reader, is complete.
+      {
         uint32_t wk[D * BITS / 32], op[D / 4];
         load_code_row<BITS, D>(stage + SP::K_OFF + code_row, wk);
         if constexpr (ODD) expand_words_v<BITS, D>(wk, op);
@@ -303,20 +278,8 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       tc_fence_before();
       named_arrive(K_READY<G> + wg, 160);
       if (pending) accumulate();
-      // ---- V row(s) -> the group's 128-byte-swizzled shared-memory stage (the PV MMA's A
-      // operand), laid out like the K row
-      if constexpr (SP::PAIR) {
-#pragma unroll 1
-        for (int u = 0; u < 2; ++u) {
-          uint32_t wv[64 * BITS / 32], op[16];
-          load_code_row<BITS, 64>(stage + SP::V_OFF + u * TILE * SP::RB + code_row, wv);
-          expand_words_v<BITS, 64>(wv, op);
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc)
-            st_shared_v4((v_row ^ (u << 6)) ^ (cc << 4), op[4 * cc], op[4 * cc + 1], op[4 * cc + 2],
-                         op[4 * cc + 3]);
-        }
-      } else {
+      // ---- V row -> the group's 128-byte-swizzled shared-memory stage (the PV MMA's A operand)
+      {
         uint32_t wv[D * BITS / 32], op[D / 4];
         load_code_row<BITS, D>(stage + SP::V_OFF + code_row, wv);
         expand_words_v<BITS, D>(wv, op);
@@ -324,33 +287,27 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         for (int cc = 0; cc < D / 16; ++cc)
           st_shared_v4(v_row ^ (cc << 4), op[4 * cc], op[4 * cc + 1], op[4 * cc + 2], op[4 * cc + 3]);
       }
-      // the tokens' records; then the ring stage goes back to the producers
-      float sk[NT], zk[NT], sv[NT], zv[NT];
-      float sk1[NT] = {}, zk1[NT] = {};   // the second K group's pair (KG == 2)
-#pragma unroll
-      for (int u = 0; u < NT; ++u) {
-        const int row = u * TILE + t;
-        if constexpr (KG == 2) {   // K ring: (s, z) of both groups; V ring after the page's K ring
-          uint32_t k0, k1, vr;
-          const uint32_t slot = stage + SP::S_OFF + (row >> 6) * SP::SCALE_PAGE;
-          asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(k0), "=r"(k1)
-                       : "r"(slot + (row & 63) * 8));
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(vr) : "r"(slot + 8 * PAGE + (row & 63) * 4));
-          sk[u] = __uint_as_float(k0 << 16); zk[u] = __uint_as_float(k0 & 0xFFFF0000u);
-          sk1[u] = __uint_as_float(k1 << 16); zk1[u] = __uint_as_float(k1 & 0xFFFF0000u);
-          sv[u] = __uint_as_float(vr << 16); zv[u] = __uint_as_float(vr & 0xFFFF0000u);
-        } else if constexpr (KG != 3) {   // KG == 1: f32 records; KG == 3: bf16 pairs
-          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
-                       : "=f"(sk[u]), "=f"(zk[u]), "=f"(sv[u]), "=f"(zv[u])
-                       : "r"(stage + SP::S_OFF + row * 16));
-        } else {   // (s, z) as bf16 pairs, 8 bytes a token, each page at its f32-sized slot
-          uint32_t kr, vr;
-          asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];"
-                       : "=r"(kr), "=r"(vr)
-                       : "r"(stage + SP::S_OFF + (row >> 6) * SP::SCALE_PAGE + (row & 63) * 8));
-          sk[u] = __uint_as_float(kr << 16); zk[u] = __uint_as_float(kr & 0xFFFF0000u);
-          sv[u] = __uint_as_float(vr << 16); zv[u] = __uint_as_float(vr & 0xFFFF0000u);
-        }
+      // the token's record; then the ring stage goes back to the producers
+      float sk, zk, sv, zv;
+      float sk1 = 0.f, zk1 = 0.f;         // the second K group's pair (KG == 2)
+      if constexpr (KG == 2) {            // K ring: (s, z) of both groups; V ring after the page's K ring
+        uint32_t k0, k1, vr;
+        const uint32_t slot = stage + SP::S_OFF + (t >> 6) * SP::SCALE_PAGE;
+        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(k0), "=r"(k1)
+                     : "r"(slot + (t & 63) * 8));
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(vr) : "r"(slot + 8 * PAGE + (t & 63) * 4));
+        sk = __uint_as_float(k0 << 16); zk = __uint_as_float(k0 & 0xFFFF0000u);
+        sk1 = __uint_as_float(k1 << 16); zk1 = __uint_as_float(k1 & 0xFFFF0000u);
+        sv = __uint_as_float(vr << 16); zv = __uint_as_float(vr & 0xFFFF0000u);
+      } else if constexpr (KG != 3) {     // KG == 1: f32 records; KG == 3: bf16 pairs
+        ld_shared_f4(stage + SP::S_OFF + t * 16, sk, zk, sv, zv);
+      } else {   // (s, z) as bf16 pairs, 8 bytes a token, each page at its f32-sized slot
+        uint32_t kr, vr;
+        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];"
+                     : "=r"(kr), "=r"(vr)
+                     : "r"(stage + SP::S_OFF + (t >> 6) * SP::SCALE_PAGE + (t & 63) * 8));
+        sk = __uint_as_float(kr << 16); zk = __uint_as_float(kr & 0xFFFF0000u);
+        sv = __uint_as_float(vr << 16); zv = __uint_as_float(vr & 0xFFFF0000u);
       }
       __syncwarp();
       mbar_arrive_elect(full + 8 * NS);   // ring_empty of the stage
@@ -361,23 +318,21 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         full -= 8 * NS;
         ring_ph ^= 1u;
       }
-      // ---- raw scores: columns [0, GP) for the lane's first token, [8, 8 + GP) for its second
+      // ---- raw scores: columns [0, GP), and [8, 8 + GP) where the rows' halves are split
       mbar_wait_warp(bars.s_done(wg), ph, abort_flag, status);
       tc_fence_after();
-      constexpr int RS = 8;
-      uint32_t raw[(NT == 2 || KG == 2 || ODD) ? 16 : GP];
-      if constexpr (NT == 2 || KG == 2 || ODD) tmem_ld16(s_src, raw);
+      uint32_t raw[(KG == 2 || ODD) ? 16 : GP];
+      if constexpr (KG == 2 || ODD) tmem_ld16(s_src, raw);
       else if constexpr (GP == 4) tmem_ld4(s_src, raw);
       else tmem_ld8(s_src, raw);
       tmem_ld_wait();
-      uint32_t pw[NT][4];
       // Only a request's last tile has positions past its length: their scores become -inf and
       // their records are neutralised, so stale shared memory can never reach the output.
       // Scores are taken relative to the group's running reference m, which may lag the true
       // maximum by up to MAX_LAG (p <= 2^MAX_LAG; the P scale leaves that headroom below the E4M3
       // range). Only when some score of the tile exceeds that does the group exchange the exact
       // column maxima and rescale; the common tile costs one reducing barrier.
-      float x[NT][GP], wsc[NT];
+      float x[GP];
       float over = -INFINITY;
       // with several query tokens a column stops short of the request's last positions
       const bool inside = pos0 <= whole;   // (the same for the whole group)
@@ -387,33 +342,30 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         ld_shared_f4(smem_u32(head_k + h), hk[h], hk[h + 1], hk[h + 2], hk[h + 3]);
         ld_shared_f4(smem_u32(head_k + 8 + h), hz[h], hz[h + 1], hz[h + 2], hz[h + 3]);
       }
+      const bool valid = inside || pos0 < w.len;
+      float wsc = sv * p2lp;
+      if (!valid) { wsc = 0.f; zv = 0.f; }
 #pragma unroll
-      for (int u = 0; u < NT; ++u) {
-        const bool valid = inside || pos0 + u * TILE < w.len;
-        wsc[u] = sv[u] * p2lp;
-        if (!valid) { wsc[u] = 0.f; zv[u] = 0.f; }
-#pragma unroll
-        for (int h = 0; h < GP; ++h) {
-          float xv, s = __uint_as_float(raw[RS * u + h]);
-          if constexpr (ODD) s = fmaf(0.25f, __uint_as_float(raw[8 + h]), s);
-          if constexpr (KG == 2)
-            xv = fmaf(hk[h] * sk[u], s,
-                      fmaf(hk[h] * sk1[u], __uint_as_float(raw[RS * u + 8 + h]),
-                           fmaf(hz[h], zk[u], fmaf(head_k[16 + h], zk1[u], -m[h]))));
-          else
-            xv = fmaf(hk[h] * sk[u], s, fmaf(hz[h], zk[u], -m[h]));
-          x[u][h] = valid ? xv : -INFINITY;
-          over = fmaxf(over, x[u][h]);
-        }
+      for (int h = 0; h < GP; ++h) {
+        float xv, s = __uint_as_float(raw[h]);
+        if constexpr (ODD) s = fmaf(0.25f, __uint_as_float(raw[8 + h]), s);
+        if constexpr (KG == 2)
+          xv = fmaf(hk[h] * sk, s,
+                    fmaf(hk[h] * sk1, __uint_as_float(raw[8 + h]),
+                         fmaf(hz[h], zk, fmaf(head_k[16 + h], zk1, -m[h]))));
+        else
+          xv = fmaf(hk[h] * sk, s, fmaf(hz[h], zk, -m[h]));
+        x[h] = valid ? xv : -INFINITY;
+        over = fmaxf(over, x[h]);
       }
       if constexpr (MQ) {
-        if (!inside) mask_lagged_columns<NT, GP>(P, w.len, w.ht, pos0, TILE, x, over);
+        if (!inside) mask_lagged_columns<GP>(P, w.len, w.ht, pos0, x, over);
       }
       if (named_barrier_or(1 + wg, 128, over > (unset ? -INFINITY : MAX_LAG))) {
         float* wmax = red_max + ((wg * 2 + ph) * 4 + wq) * 8;
 #pragma unroll
         for (int h = 0; h < GP; ++h) {
-          const float wm = warp_max_f32(NT == 2 ? fmaxf(x[0][h], x[NT - 1][h]) : x[0][h]);
+          const float wm = warp_max_f32(x[h]);
           if (lane == 0) wmax[h] = wm;
         }
         named_barrier(1 + wg, 128);
@@ -431,37 +383,31 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
             l[h] *= corr;
             c[h] *= corr;
             oacc[h] *= corr;   // holds every earlier tile's O (added above)
-#pragma unroll
-            for (int u = 0; u < NT; ++u) x[u][h] -= delta;
+            x[h] -= delta;
           }
         }
       }
       // p = 2^x, w = p * s_v 2^lp, four heads at a time as E4M3 hi + lo/16. (ex2 on f32: the
       // f16x2 form takes twice as long per instruction on this part, so it saves nothing.)
+      uint32_t pw[4] = {};
 #pragma unroll
-      for (int u = 0; u < NT; ++u) {
+      for (int h = 0; h < GP; h += 4) {
+        __half2 w2[2];
 #pragma unroll
-        for (int h = 0; h < GP; h += 4) {
-          __half2 w2[2];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int a = h + 2 * i;
-            const float p0 = fast_exp2(x[u][a]), p1 = fast_exp2(x[u][a + 1]);
-            l[a] += p0;
-            l[a + 1] += p1;
-            c[a] = fmaf(p0, zv[u], c[a]);
-            c[a + 1] = fmaf(p1, zv[u], c[a + 1]);
-            w2[i] = __floats2half2_rn(p0 * wsc[u], p1 * wsc[u]);
-          }
-          split_e4m3x4(w2[0], w2[1], pw[u][h >> 2], pw[u][2 + (h >> 2)]);
+        for (int i = 0; i < 2; ++i) {
+          const int a = h + 2 * i;
+          const float p0 = fast_exp2(x[a]), p1 = fast_exp2(x[a + 1]);
+          l[a] += p0;
+          l[a + 1] += p1;
+          c[a] = fmaf(p0, zv, c[a]);
+          c[a + 1] = fmaf(p1, zv, c[a + 1]);
+          w2[i] = __floats2half2_rn(p0 * wsc, p1 * wsc);
         }
-        if constexpr (GP == 4) pw[u][1] = pw[u][3] = 0u;
+        split_e4m3x4(w2[0], w2[1], pw[h >> 2], pw[2 + (h >> 2)]);
       }
-      // the P row(s): bytes [hi_0..hi_7 | lo_0..lo_7], one plane of 128 rows per token of a lane;
-      // with the V rows above they complete the PV MMA's operands
-#pragma unroll
-      for (int u = 0; u < NT; ++u)
-        st_shared_v4(p_row + u * TILE * 16, pw[u][0], pw[u][1], pw[u][2], pw[u][3]);
+      // the P row: bytes [hi_0..hi_7 | lo_0..lo_7]; with the V rows above they complete the PV MMA's
+      // operands
+      st_shared_v4(p_row, pw[0], pw[1], pw[2], pw[3]);
       fence_proxy_async();
       tc_fence_before();   // (orders the O read above before the PV MMA)
       __syncwarp();
@@ -531,9 +477,7 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
                                                            g * SP::XCHG_STRIDE);
           const float* xmeta = xo + TILE * 8;
           const float m1 = xmeta[h], l1 = xmeta[8 + h], c1 = xmeta[16 + h];
-          // at two tokens per lane, channel t's sum is split over rows t and t + 64
-          float o1 = xo[h * TILE + t];
-          if (SP::PAIR && t < 64) o1 += xo[h * TILE + t + 64];
+          const float o1 = xo[h * TILE + t];
           const float Mn = fmaxf(M, m1);
           const float f0 = M == -INFINITY ? 0.f : exp2f(M - Mn);
           const float f1 = m1 == -INFINITY ? 0.f : exp2f(m1 - Mn);
@@ -573,7 +517,6 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
     // are next written after the next item's first all-group barrier, which this read precedes)
     if (w.slot != -2) {
       const int ch = channel_of_expanded_pos<BITS>(t);
-      const bool on = t < D;   // head_dim 64: the upper half of the O rows is padding
 #pragma unroll
       for (int i = 0; i < HPG; ++i) {
         const int h = wg + i * G;
@@ -585,13 +528,13 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
         if (w.slot < 0) {
           const long long orow = caller_row<MQ>(P, w.b, w.kvh, hl);
           const float val = L > 0.f ? O / L * P.a.o_scale : 0.f;
-          if (on) store_value(P.a.out, P.a.out_dtype, orow * D + ch, val);
+          store_value(P.a.out, P.a.out_dtype, orow * D + ch, val);
           if (t == 0 && P.a.lse != nullptr)
             P.a.lse[orow] = L > 0.f ? (M + log2f(L)) * LN2 : -INFINITY;
         } else {
           const long long prow =
               static_cast<long long>(w.slot) * P.a.batch * P.a.num_qo_heads + row;
-          if (on) P.a.o_partial[prow * D + ch] = O;
+          P.a.o_partial[prow * D + ch] = O;
           if (t == 0) { P.a.l_partial[prow] = L; P.a.m_partial[prow] = M; }
         }
       }
@@ -630,18 +573,16 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
 }  // namespace
 
 template <int BITS, int D, int GP, int KG, bool MQ>
-__global__ void __launch_bounds__(decode_threads(BITS, D), 1)
+__global__ void __launch_bounds__(DECODE_THREADS, 1)
 decode_kernel(const __grid_constant__ DecodeParams P) {
   // KG: 1 whole-head K with f32 records, 3 the same with bf16 pairs, 2 two 64-channel K groups
-  static_assert(KG == 1 || KG == 3 || (KG == 2 && D == 128),
-                "K groups of 64 channels at head_dim 128");
-  static_assert(D == 64 || D == 128, "this build tiles head_dim 64 and 128");
+  static_assert(KG >= 1 && KG <= 3 && D == 128, "head_dim 128");
   using SP = SmemPlan<BITS, D>;
   using TP = TmemPlan<BITS, D>;
   constexpr int G = SP::G, NS = SP::NS;
   constexpr int W_PRODUCER = 4 * G, W_S = W_PRODUCER + 1, W_PV = W_PRODUCER + 2,
                 W_PRODUCER2 = W_PRODUCER + 3;
-  static_assert(decode_threads(BITS, D) == 32 * (W_PRODUCER2 + 1), "warp roles and block size disagree");
+  static_assert(DECODE_THREADS == 32 * (W_PRODUCER2 + 1), "warp roles and block size disagree");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem = smem_raw + (smem0 - smem_u32(smem_raw));
@@ -749,23 +690,20 @@ decode_kernel(const __grid_constant__ DecodeParams P) {
           const int chunk = lane + 32 * j;      // 16 rows of eight 16-byte chunks
           const int r = chunk >> 3, cc = chunk & 7;
           uint4 v = make_uint4(0, 0, 0, 0);
-          // At two tokens per lane rows 0-7 carry the heads against the first token's half of
-          // the K row (bytes 0-63) and rows 8-15 the same heads against the second's (64-127).
-          // With two K groups of 64 channels (one token per lane) the same split of the rows
-          // yields each group's partial product in its own S column.
+          // With two K groups of 64 channels rows 0-7 carry the heads against the first group's
+          // half of the K row (bytes 0-63) and rows 8-15 the same heads against the second's.
           // INT2 with whole-head K: rows 0-7 carry the heads against the even operand words, rows
           // 8-15 the same heads against the odd ones, which hold 4 * code (expand_words_v).
-          constexpr bool SPLIT = SP::PAIR || KG == 2, ODD = odd_columns(BITS, D, KG);
+          constexpr bool SPLIT = KG == 2, ODD = odd_columns(BITS, D, KG);
           const int hl = w.ht * 8 + (r & 7);        // head inside the KV head's group
           const bool live = (SPLIT || ODD || r < 8) && hl < P.heads_per_kv;
           const long long qrow = live ? caller_row<MQ>(P, w.b, w.kvh, hl) : 0;
-          const bool mine = SPLIT ? ((r < 8) == (cc < 4)) : 16 * cc < D;
-          const int src = SP::PAIR ? (cc & 3) : cc;
+          const bool mine = !SPLIT || (r < 8) == (cc < 4);
           float qsum = 0.f;
           if (live && mine) {
             const uint4 in = __ldg(reinterpret_cast<const uint4*>(
                 static_cast<const uint8_t*>(P.a.q) +
-                qrow * D + 16 * src));
+                qrow * D + 16 * cc));
             const uint32_t words[4] = {in.x, in.y, in.z, in.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -907,11 +845,7 @@ decode_kernel(const __grid_constant__ DecodeParams P) {
         const uint32_t v_lo = v_lo0 + g * (SP::VOP_STAGE >> 4);
         const uint32_t p_lo = p_lo0 + g * (SP::P_BYTES >> 4);
         const uint32_t od = tmem + TP::O + g * TP::O_COLS;
-        // one accumulator per token of a lane: the same V rows against that token's P plane
         umma_ss_chain4<V_HI, P_HI, IDESC_PV, (32 * SP::ROW >> 4), (32 * 16 >> 4)>(od, v_lo, p_lo);
-        if constexpr (SP::PAIR)
-          umma_ss_chain4<V_HI, P_HI, IDESC_PV, (32 * SP::ROW >> 4), (32 * 16 >> 4)>(
-              od + 16, v_lo, p_lo + (TILE * 16 >> 4));
         tc_commit_elect(bars.pv_done(g));
         if (++g == G) { g = 0; gph ^= 1u; }
       }
@@ -1056,7 +990,7 @@ static int device_sm_count() {
 template <int BITS, int D, int GP, int KG = 1, bool MQ = false>
 static int launch_decode(DecodeParams& P, cudaStream_t stream) {
   using SP = SmemPlan<BITS, D>;
-  constexpr int THREADS = decode_threads(BITS, D), LIMIT = SMEM_LIMIT;
+  constexpr int THREADS = DECODE_THREADS, LIMIT = SMEM_LIMIT;
   P.ring_stages = SP::NS;
   P.tile_tokens = SP::TT;
   P.wait_budget = P.a.wait_budget_cycles > 0 ? P.a.wait_budget_cycles : WAIT_BUDGET_CYCLES;
@@ -1167,6 +1101,10 @@ extern "C" int fq_decode(const fq_pools* pools, const fq_decode_args* args, void
   const int gp = std::min(P.heads_per_kv, 8) <= 4 ? 4 : 8;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (pools->head_dim == 256) return launch_decode_wide(P, s);
+  if (pools->head_dim == 64) {
+    if (pools->k_groups != 1) return FQ_ERR_UNSUPPORTED;
+    return launch_decode_stream(P, std::min(P.heads_per_kv, 8), s);
+  }
 #define FQ_DISPATCH(DD, KK, MM)                                                               \
   do {                                                                                        \
     if (pools->bits == 2)                                                                     \
@@ -1179,18 +1117,10 @@ extern "C" int fq_decode(const fq_pools* pools, const fq_decode_args* args, void
   // records), so that the one-token builds stay as they are
   if (P.q_len > 1) {
     if (pools->k_groups != 1) return FQ_ERR_UNSUPPORTED;
-    if (pools->head_dim == 64) {
-      if (pools->scale_bf16) FQ_DISPATCH(64, 3, true);
-      FQ_DISPATCH(64, 1, true);
-    }
     if (pools->scale_bf16) FQ_DISPATCH(128, 3, true);
     FQ_DISPATCH(128, 1, true);
   }
   if (pools->k_groups == 2) FQ_DISPATCH(128, 2, false);
-  if (pools->head_dim == 64) {
-    if (pools->scale_bf16) FQ_DISPATCH(64, 3, false);
-    FQ_DISPATCH(64, 1, false);
-  }
   if (pools->scale_bf16) FQ_DISPATCH(128, 3, false);
   FQ_DISPATCH(128, 1, false);
 #undef FQ_DISPATCH

@@ -6,17 +6,13 @@
 namespace fq {
 
 constexpr int TILE = 128;            // MMA rows: tensor-memory lanes, threads of a worker group
-// Tokens per sequence tile. head_dim 128 and 256: one token per lane (two pages). head_dim 64: two
-// tokens per lane, t and 128 + t of the tile (four pages): their 64-byte operand rows sit side by
-// side in one 128-byte row, so a tile of 256 tokens costs what a 128-token tile of head_dim 128
-// costs.
+// Tokens per sequence tile, the unit the planners cut requests in: an MMA's 128 rows at head_dim 128
+// and 256, 256 at head_dim 64 (half the bytes a token).
 __host__ __device__ constexpr int tile_tokens(int, int head_dim) { return head_dim == 64 ? 256 : 128; }
 constexpr int WORK_WORDS = 8;        // int32 words per explicit work-list row
 // Worker groups of 128 threads, tile i -> group i % G; with them two producers and two MMA issuers.
-__host__ __device__ constexpr int worker_groups(int bits, int head_dim) { return 4; }
-__host__ __device__ constexpr int decode_threads(int bits, int head_dim) {
-  return 32 * (4 * worker_groups(bits, head_dim) + 4);
-}
+constexpr int WORKER_GROUPS = 4;
+constexpr int DECODE_THREADS = 32 * (4 * WORKER_GROUPS + 4);
 constexpr int SMEM_LIMIT = 232448;   // 227 KiB opt-in limit per CTA on sm_100
 struct DecodeParams {
   fq_pools p;
@@ -94,15 +90,13 @@ struct SmemPlan {
     return CHUNKS == 4 ? (row >> 1) & 3 : (CHUNKS == 2 ? (row >> 2) & 1 : 0);
   }
   static constexpr int TT = tile_tokens(BITS, D);      // tokens per tile
-  static constexpr int G = worker_groups(BITS, D);
-  static constexpr bool PAIR = D == 64;                // two tokens per lane, rows side by side
+  static constexpr int G = WORKER_GROUPS;
   static constexpr int PPT = TT / PAGE;                // pages per tile
   static constexpr int K_OFF = 0;                      // a ring stage: K pages, V pages, records
   static constexpr int V_OFF = PPT * CODE_PAGE;
   static constexpr int S_OFF = 2 * PPT * CODE_PAGE;
   static constexpr int STAGE = 2 * PPT * CODE_PAGE + PPT * SCALE_PAGE;
-  // Operand rows keep a 128-byte pitch (the swizzle atom) whatever D <= 128: head_dim 64 uses
-  // the first half of each row.
+  // Operand rows have a 128-byte pitch (the swizzle atom)
   static constexpr int ROW = 128;
   static constexpr int VOP_STAGE = TILE * ROW;   // expanded V operand, one tile
   static constexpr int Q_BYTES = 16 * ROW;             // 16 MMA rows
@@ -224,6 +218,8 @@ __device__ __forceinline__ WorkItem item_at(const DecodeParams& P, const WorkIte
 }
 // Launch of the head_dim 256 build (decode_wide.cu), called by fq_decode with checked arguments.
 int launch_decode_wide(DecodeParams& P, cudaStream_t stream);
+// Launch of the head_dim 64 build (decode_stream.cu), likewise.
+int launch_decode_stream(DecodeParams& P, int columns, cudaStream_t stream);
 
 __device__ inline ItemRange item_range(const DecodeParams& P) {
   if (P.a.worklist == nullptr)
@@ -385,7 +381,7 @@ static __device__ __noinline__ void merge_unit_partials(const DecodeParams& P, i
       }
     // With several heads at a time (the head_dim 256 kernel) the first eight slots' o values are
     // requested together with the (m, l) pairs: a unit of up to eight pieces then costs one
-    // memory round trip, not two in sequence. In the head_dim 64/128 kernel the same order
+    // memory round trip, not two in sequence. In the head_dim 128 kernel the same order
     // measured 1 to 3 % slower on its many-item workload (register allocation of the kernel
     // around this out-of-line function), so there the fetch stays inside the loop.
     constexpr bool EARLY = HU > 1;
