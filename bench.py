@@ -817,7 +817,8 @@ def main():
                          "traffic_from": "a separate ncu capture of this command's decode launch "
                                          "(dram__bytes_read.sum + dram__bytes_write.sum), not "
                                          "measured by this run" if default_args else None,
-                         "kernel": "decode_wide_kernel" if cfg["d"] == 256 else "decode_kernel",
+                         "kernel": {64: "stream_decode_kernel", 256: "decode_wide_kernel"}.get(
+                             cfg["d"], "decode_kernel"),
                          "kernel_us": decode_ms * 1e3,
                          "algorithmic_bytes": abytes, "frac_of_8tbs_nominal": achieved / 8000.0},
             "e2e": {"value": world * b * args.q_len / (e2e_ms * 1e-3), "unit": "tokens/s",

@@ -1,6 +1,6 @@
 // Paged GQA decode attention over packed INT2/INT4 KV at head_dim 256, sm_100a.
 //
-// Same arithmetic as the head_dim 64/128 kernel (decode.cu; reference semantics
+// Same arithmetic as the head_dim 128 kernel (decode.cu; reference semantics
 // src/foscar/wrapper.py:1153-1171, fold algebra src/foscar/_sm100/int_fold_decode.py:5-22,
 // 378-434; the reference tiles head_dim 256 as two K/V boxes per page,
 // src/foscar/_sm100/int_fold_decode.py:1509-1530, 3316-3413). A token's operand row is 256 bytes,
