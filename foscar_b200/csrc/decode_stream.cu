@@ -48,9 +48,11 @@ namespace stream {
 namespace {
 
 constexpr int CHUNK = 32;          // tokens of a chunk
-// A warp's chunks looked up ahead: a ring of {page id, 2 * KV head + page half}, then what the
-// lanes remember of their walks over the items.
+// A warp's chunks looked up ahead: a ring of {page id, 2 * KV head + page half}, or {-1, NO_CHUNK}:
+// no such chunk, or nothing valid in it (the page id is the caller's word as it stands, so no value
+// of it can be the mark); then what the lanes remember of their walks over the items.
 constexpr int AHEAD = 64;
+constexpr int NO_CHUNK = -1;
 constexpr int TABLE_BYTES = AHEAD * 8 + 32 * 12;
 constexpr int SLOTS = 32;          // items that may be waiting for their last warps, by item % SLOTS
 // A head's running reference may lag the true maximum by up to MAX_LAG (log2 units); when it is
@@ -284,8 +286,7 @@ __device__ __forceinline__ int chunks_of(const WorkItem& w, int tile) {
 // chunk and has the page id copied to the chunk's table entry (asynchronously: it has landed when
 // the copies of the chunk being issued have). Out of line, with the walks in shared memory, so
 // that the chunk loop holds none of it in registers.
-// Entry: {page id, 2 * KV head + page half}; -1: no such chunk, or nothing valid in it; -2: the
-// page table has no entry for it.
+// A chunk that the page table has no entry for gets -1, like any page id outside the pool.
 __device__ __noinline__ void look_up_chunks(const DecodeParams& P, const WorkItem* cached,
                                             const WorkItem* more, int slots, const ItemRange items,
                                             int warps, uint8_t* table, int at, int from, int to) {
@@ -294,7 +295,7 @@ __device__ __noinline__ void look_up_chunks(const DecodeParams& P, const WorkIte
     int* const walk = reinterpret_cast<int*>(table + AHEAD * 8) + 3 * lane;
     int k = walk[0], base = walk[1];
     const int g = walk[2];
-    int2 entry = make_int2(-1, 0);
+    int half = NO_CHUNK;
     int2* const place = reinterpret_cast<int2*>(table) + ((at + lane) & (AHEAD - 1));
     for (int wi = items.begin + k * items.step; wi < items.end; wi += items.step, ++k) {
       const WorkItem w = item_at(P, cached, more, slots, k, wi);
@@ -305,22 +306,21 @@ __device__ __noinline__ void look_up_chunks(const DecodeParams& P, const WorkIte
       }
       const int pos = w.t0 * P.tile_tokens + CHUNK * (g - base);
       if (pos < min(w.t1 * P.tile_tokens, w.len)) {
-        entry.y = 2 * w.kvh + (pos & (PAGE - 1)) / CHUNK;
+        half = 2 * w.kvh + (pos & (PAGE - 1)) / CHUNK;
         const long long e = static_cast<long long>(w.table_off) + pos / PAGE;
         if (e >= 0 && e < P.a.table_len)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(place)),
                        "l"(P.a.page_table + e) : "memory");
         else
-          place->x = -2;
-        entry.x = -3;
+          place->x = -1;
       }
       break;
     }
     walk[0] = k;
     walk[1] = base;
     walk[2] = g + 32 * warps;
-    if (entry.x == -1) place->x = -1;
-    place->y = entry.y;
+    if (half == NO_CHUNK) place->x = -1;
+    place->y = half;
   }
 }
 
@@ -455,7 +455,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
           cp_async16_stream(dst + SP::R_OFF + 16 * lane,
                             ss + (8 * PAGE - 256) + half * (4 * CHUNK), stream_policy);
       }
-    } else if (entry.x != -1) {
+    } else if (entry.y != NO_CHUNK) {   // (no chunk: nothing to copy)
       bad_page(issue_to + SP::R_OFF, status);
     }
     cp_async_commit();

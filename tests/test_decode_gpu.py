@@ -356,3 +356,37 @@ def test_bad_page_id_sets_status_without_fault():
     w.run(make_q(1, 8, 128), cache, out=out)
     torch.cuda.synchronize()
     assert w.last_status() & 0x2
+
+
+@pytest.mark.parametrize("bits", [2, 4])
+@pytest.mark.parametrize("d,hq,hkv", [(64, 16, 2), (64, 8, 2), (128, 8, 2), (256, 8, 2)])
+@pytest.mark.parametrize("bad", [-1, -5, 2**31 - 1, "pool size"])
+def test_every_bad_page_id_is_reported(bits, d, hq, hkv, bad):
+    """A page id outside the pool in the middle of a request or at its end, the usual padding value
+    -1 among them: the status bit is set, and the other requests' rows are those of the good table,
+    bit for bit (which are the oracle's)."""
+    from foscar_b200 import PagedDecodeWrapper, QuantKVLayout
+    seq = [700, 256, 90]
+    indptr, indices, slots, npages = paged_batch(seq, seed=41)
+    layout = QuantKVLayout.create(bits=bits, head_dim=d, num_kv_heads=hkv, device="cuda")
+    cache = layout.allocate(npages)
+    k, v = make_kv(len(slots), hkv, d, seed=41)
+    cache.append(k, v, torch.from_numpy(slots).cuda())
+    q = make_q(len(seq), hq, d, seed=42)
+    outs = []
+    for spoilt in ((), (1,), (3,), (0, 1, 2, 3)):     # entries of the second request's table
+        table = indices.copy()
+        for e in spoilt:
+            table[indptr[1] + e] = npages if bad == "pool size" else bad
+        w = PagedDecodeWrapper(torch.empty(16 << 20, dtype=torch.uint8, device="cuda"))
+        w.plan(torch.from_numpy(indptr), torch.from_numpy(table).cuda(),
+               torch.tensor(seq, dtype=torch.int32), hq, layout)
+        outs.append(w.run(q, cache))
+        torch.cuda.synchronize()
+        assert w.last_status() == (0x2 if spoilt else 0)
+    pools = cpu_twin(cache, k, v, slots)
+    want, _ = oracle_outputs(pools, q.cpu(), indptr, indices, seq, d ** -0.5)
+    for b in (0, 2):
+        assert (outs[0][b].float().cpu() - want[b]).abs().max().item() <= MAX_ABS
+        for out in outs[1:]:
+            assert torch.equal(out[b], outs[0][b])
