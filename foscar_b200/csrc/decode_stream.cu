@@ -596,6 +596,11 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
     float* const mine = reinterpret_cast<float*>(smem + SP::STATE_OFF + warp * SP::STATE);
     warp_wait<false>(ctl + CTL_BUSY + warp, 0, abort_flag, status);
     bool last = true;
+    // The items of a slot complete in turn: DONE[slot] counts them, and one that counts its parts in,
+    // or itself done, waits for all the slot's earlier items first. (That holds for an item of one
+    // part too: its early count would pass for an earlier item that is still open, and the item
+    // between them would then count on that one's parts. It waits for earlier items only, so the
+    // waits end.)
     if (parts > 1) {
 #pragma unroll
       for (int q = 0; q < SP::NST / 4; ++q)
@@ -610,7 +615,6 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
           meta[16 + h0 + i] = c[i];
         }
       if (lane == 0) ctl[CTL_BUSY + warp] = 1;
-      // an earlier item of the same slot must be complete before this one counts there
       warp_wait<true>(ctl + CTL_DONE + slot, c_k / SLOTS, abort_flag, status);
       __threadfence_block();
       int seen = 0;
@@ -661,8 +665,9 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
           atomicAdd(const_cast<int*>(ctl) + CTL_DONE + slot, 1);
         }
       }
-    } else if (lane == 0) {
-      atomicAdd(const_cast<int*>(ctl) + CTL_DONE + slot, 1);
+    } else {
+      warp_wait<true>(ctl + CTL_DONE + slot, c_k / SLOTS, abort_flag, status);
+      if (lane == 0) atomicAdd(const_cast<int*>(ctl) + CTL_DONE + slot, 1);
     }
     if (!last) return;
     if (w.slot != -2) {

@@ -303,6 +303,60 @@ def test_many_single_tile_items(bits, d):
         assert err.max().item() <= MAX_ABS, (b, err.max().item())
 
 
+def _short_and_long(n, longest, at, rng):
+    """n requests of 1 to 64 tokens with long ones among them."""
+    seq = [int(x) for x in rng.integers(1, 65, n)]
+    for i, b in enumerate(at):
+        seq[b] = longest - 700 * i
+    return seq
+
+
+@pytest.mark.parametrize("bits,hq,hkv,q_len,kv_splits,ctas,n", [
+    (2, 8, 8, 1, None, None, 2048),    # a planned list, 111 items a CTA
+    (4, 64, 8, 4, None, None, 512),    # four query tokens: four head tiles, 111 items a CTA
+    (4, 16, 2, 1, 8, None, 1024),      # uniform pieces, seven of eight empty
+    (2, 8, 2, 1, 4, 5, 300),           # few CTAs: 480 items each, merges of split units all along
+    (2, 64, 8, 2, 3, 9, 100),
+])
+def test_head_dim_64_many_items_a_cta(bits, hq, hkv, q_len, kv_splits, ctas, n):
+    """Far more work items on a CTA than it keeps open at a time (32), most of them one 32-token
+    chunk, which one warp does alone, between long ones that all sixteen warps share, empty pieces
+    and split units (one warp merges those and falls behind): every row is the oracle's, and the
+    launch repeats itself bit by bit."""
+    from foscar_b200 import PagedDecodeWrapper, QuantKVLayout
+    d = 64
+    seq = _short_and_long(n, 9000, (0, n // 3, n // 2, n - 1), np.random.default_rng(n))
+    seq = [max(s, q_len) for s in seq]
+    indptr, indices, slots, npages = paged_batch(seq, seed=n)
+    k, v = make_kv(len(slots), hkv, d, seed=n)
+    layout = QuantKVLayout.create(bits=bits, head_dim=d, num_kv_heads=hkv, device="cuda")
+    cache = layout.allocate(npages)
+    cache.append(k, v, torch.from_numpy(slots).cuda())
+    q = make_q(n * q_len, hq, d, seed=n + 1).view(n, q_len, hq, d)
+    w = PagedDecodeWrapper(torch.empty(256 << 20, dtype=torch.uint8, device="cuda"))
+    w.plan(torch.from_numpy(indptr).cuda(), torch.from_numpy(indices).cuda(),
+           torch.tensor(seq, dtype=torch.int32), hq, layout, q_len_per_req=q_len,
+           kv_splits=kv_splits)
+    if ctas is not None:        # (uniform pieces run on any number of CTAs)
+        w._plan_args = w._build_plan_args()
+        w._plan_args.max_ctas = ctas
+    first = None
+    for _ in range(20):
+        out = torch.full((n, q_len, hq, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        w.run(q, cache, out=out)
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    torch.cuda.synchronize()
+    assert w.last_status() == 0, w.last_status()
+    # (a query token that is not the request's last sees that many positions fewer)
+    pools = cpu_twin(cache, k, v, slots)
+    for l in range(q_len):
+        sees = [s - (q_len - 1 - l) for s in seq]
+        want, _ = oracle_outputs(pools, q[:, l].cpu(), indptr, indices, sees, d ** -0.5)
+        err = (out[:, l].float().cpu() - want).abs()
+        assert err.max().item() <= MAX_ABS, (l, err.max().item(), int(err.flatten(1).max(1)[0].argmax()))
+
+
 @pytest.mark.parametrize("stages", ["4", "5", "6", "7"])
 def test_shallow_rings(stages, monkeypatch):
     """The shared-memory ring at its smallest depths (the library rounds an odd request down):
