@@ -61,6 +61,7 @@ namespace {
 
 // Barrier words of a CTA, at fixed offsets: one per ring stage and direction, one per query stage
 // and direction, and per worker group
+//   k_ready : the tile's K operand is in tensor memory (the group's four warps)
 //   s_done  : the tile's S MMA is complete (commit)
 //   pv_ready: the tile's V operand and P rows are in shared memory (the group's four warps); the
 //             group has by then read the O of its previous tile
@@ -68,8 +69,11 @@ namespace {
 //             rows are free
 // A group's n-th tile uses phase n & 1. stored: every worker warp has issued its output or partial
 // stores of the work item (one phase per item): what orders a split piece's partials before its
-// count-in. That a group's K operand is in tensor memory goes from its four warps to the S issuer
-// through a named barrier of 160 threads (K_READY): one instruction a warp.
+// count-in. Every hand-off between roles is one of these words, so that its wait is bounded and a
+// role that gave up cannot keep another from ending. (Named barriers, whose waits nothing can end,
+// stay among the worker groups: those execute the same ones whatever their waits returned. With one
+// for the K operand a group that had given up could arrive twice before the issuer did once, which
+// was then a warp short for good.)
 template <int G, int NS>
 struct Bars {
   uint32_t base;
@@ -80,12 +84,11 @@ struct Bars {
   __device__ uint32_t s_done(int g) const { return base + 8u * (2 * NS + 4 + g); }
   __device__ uint32_t pv_done(int g) const { return base + 8u * (2 * NS + 4 + G + g); }
   __device__ uint32_t pv_ready(int g) const { return base + 8u * (2 * NS + 4 + 2 * G + g); }
-  __device__ uint32_t stored() const { return base + 8u * (2 * NS + 4 + 3 * G); }
-  static constexpr int WORDS = 2 * NS + 5 + 3 * G;
+  __device__ uint32_t k_ready(int g) const { return base + 8u * (2 * NS + 4 + 3 * G + g); }
+  __device__ uint32_t stored() const { return base + 8u * (2 * NS + 4 + 4 * G); }
+  static constexpr int WORDS = 2 * NS + 5 + 4 * G;
 };
-// Named barriers: 0 the CTA, 1 .. G inside a group, 1 + G all groups, then one per group for its K
-// operand (there are sixteen in all).
-template <int G> constexpr int K_READY = 2 + G;
+// Named barriers: 0 the CTA, 1 .. G inside a group, 1 + G all groups.
 
 // Tensor-memory column plan (f32 columns): per worker group one K operand stage (a 128-byte row
 // per lane), one S buffer and one O buffer of 16 columns.
@@ -276,7 +279,8 @@ __device__ __forceinline__ void worker_role(const DecodeParams& P, uint8_t* smem
       }
       tmem_st_wait();
       tc_fence_before();
-      named_arrive(K_READY<G> + wg, 160);
+      __syncwarp();
+      mbar_arrive_elect(bars.k_ready(wg));
       if (pending) accumulate();
       // ---- V row -> the group's 128-byte-swizzled shared-memory stage (the PV MMA's A operand)
       {
@@ -601,6 +605,7 @@ decode_kernel(const __grid_constant__ DecodeParams P) {
       mbar_init(bars.ring_empty(s), 4);  // the four warps of the group that took the tile
     }
     for (int g = 0; g < G; ++g) {
+      mbar_init(bars.k_ready(g), 4);
       mbar_init(bars.s_done(g), 1);
       mbar_init(bars.pv_done(g), 1);
       mbar_init(bars.pv_ready(g), 4);
@@ -811,6 +816,7 @@ decode_kernel(const __grid_constant__ DecodeParams P) {
     constexpr uint32_t IDESC_S = make_idesc_e4m3(128, 16, 0, 0);
     constexpr uint32_t Q_HI = smem_desc_hi(1024, 2);
     int qi = 0, g = 0;   // tiles go to the groups in turn
+    uint32_t gph = 0;    // phase of the groups' barriers: flips once per round of G tiles
     for (int wi = items.begin, ik = 0; wi < items.end; wi += items.step, ++ik) {
       const WorkItem w = uniform_item(item_at(P, item_cache, item_more, SP::ITEM_SLOTS, ik, wi));
       if (w.t1 <= w.t0) continue;
@@ -819,11 +825,11 @@ decode_kernel(const __grid_constant__ DecodeParams P) {
       const uint32_t q_lo = smem_desc_lo(smem0 + SP::Q_OFF + qb * SP::Q_BYTES, 16);
 #pragma unroll 1
       for (int t = w.t0; t < w.t1; ++t) {
-        named_barrier(K_READY<G> + g, 160);
+        mbar_wait_warp(bars.k_ready(g), gph, abort_flag, status);
         tc_fence_after();
         umma_ts_chain4<Q_HI, IDESC_S>(tmem + TP::S + g * TP::S_COLS, tmem + TP::KOP + g * TP::KOP_COLS,
                                       q_lo, bars.s_done(g));
-        if (++g == G) g = 0;
+        if (++g == G) { g = 0; gph ^= 1u; }
       }
       tc_commit_elect(bars.q_empty(qb));   // after the item's last chain
       ++qi;
@@ -948,26 +954,40 @@ umma_selftest_kernel(int mode, const uint8_t* k_bytes, const uint8_t* q_bytes,
   }
 }
 
-// Wait self test (see foscar_b200.h): every thread waits, with the given cycle budget, for a
-// barrier phase that nothing completes. The first waiter to run out raises the CTA's abort flag
+// Wait self test (see foscar_b200.h): every form of wait that the decode kernels' roles use, one
+// after the other, each with the given cycle budget and for something that never comes: a barrier
+// phase that nothing completes, waited for by single threads, and a hand-off that is two of its four
+// arrivals short, waited for by whole warps. The first waiter to run out raises the CTA's abort flag
 // and FQ_STATUS_TIMEOUT; the others fall through; the kernel returns.
 __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(long long budget, int* status,
                                                               int* gave_up) {
-  __shared__ __align__(8) unsigned long long bar_word;
+  __shared__ __align__(8) unsigned long long bar_words[2];
   __shared__ __align__(8) int ctl_words[4];
   volatile int* abort_flag = ctl_words;
-  const uint32_t bar = smem_u32(&bar_word);
+  const uint32_t alone = smem_u32(&bar_words[0]), handoff = smem_u32(&bar_words[1]);
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     set_wait_budget(abort_flag, budget);
-    mbar_init(bar, 1);
+    mbar_init(alone, 1);
+    mbar_init(handoff, 4);
     fence_barrier_init();
   }
   __syncthreads();
-  mbar_wait(bar, 0, abort_flag, status);    // runs out
-  mbar_wait(bar, 0, abort_flag, status);    // returns at once: the CTA has given up
-  __syncthreads();
-  if (threadIdx.x == 0 && gave_up != nullptr) *gave_up = *abort_flag;
+  int all = 1;
+  auto next_form = [&]() {   // was the flag raised? down again for the next form
+    __syncthreads();
+    all &= *abort_flag;
+    __syncthreads();
+    if (threadIdx.x == 0) *abort_flag = 0;
+    __syncthreads();
+  };
+  mbar_wait(alone, 0, abort_flag, status);    // runs out
+  mbar_wait(alone, 0, abort_flag, status);    // returns at once: the CTA has given up
+  next_form();
+  mbar_arrive_elect(handoff);                 // (one a warp: two of four)
+  mbar_wait_warp(handoff, 0, abort_flag, status);
+  next_form();
+  if (threadIdx.x == 0 && gave_up != nullptr) *gave_up = all;
 }
 
 }  // namespace fq

@@ -287,11 +287,11 @@ int fq_umma_selftest(int32_t mode, const uint8_t* k_bytes, const uint8_t* q_byte
                      const uint8_t* v_bytes, const uint8_t* p_bytes, float* s_out, float* o_out,
                      int32_t* status, void* stream);
 
-/* Wait self test: one small kernel whose threads wait, with the given cycle budget, for a
- * barrier phase that nothing completes. The wait runs out, the kernel sets FQ_STATUS_TIMEOUT in
- * *status and 1 in *gave_up and returns; the context stays usable. It exercises the give-up path
- * every bounded device wait of this library shares (the reference traps instead,
- * src/foscar/_sm100/int_fold_decode.py:131-175). */
+/* Wait self test: one small kernel whose threads wait, with the given cycle budget for each form of
+ * wait, for barrier phases that nothing completes. Every wait runs out, the kernel sets
+ * FQ_STATUS_TIMEOUT in *status and 1 in *gave_up (0 if some form did not give up) and returns; the
+ * context stays usable. It exercises the give-up path every bounded device wait of this library
+ * shares (the reference traps instead, src/foscar/_sm100/int_fold_decode.py:131-175). */
 int fq_wait_selftest(int64_t budget_cycles, int32_t* status, int32_t* gave_up, void* stream);
 
 #ifdef __cplusplus

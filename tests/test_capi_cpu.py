@@ -31,6 +31,23 @@ def test_library_builds_loads_and_exports_the_header():
     assert lib.fq_error_string(-2).decode() == "unsupported configuration"
 
 
+def test_roles_hand_over_by_bounded_waits_only():
+    """A named barrier's wait cannot be ended by the give-up flag, so in the device code they join
+    whole worker groups (128 threads each), which execute the same ones whatever their other waits
+    returned; between roles there are mbarriers and counted words, whose waits are bounded."""
+    csrc = os.path.join(ROOT, "foscar_b200", "csrc")
+    calls = []
+    for name in sorted(os.listdir(csrc)):
+        text = re.sub(r"//.*", "", open(os.path.join(csrc, name)).read())
+        # an arrival that does not wait is a hand-off to another role
+        assert not re.search(r"\b(bar|barrier(\.cta)?)\.arrive", text), name
+        if not name.endswith(".cuh"):     # (their definitions)
+            calls += [(name, c) for c in re.findall(r"\bnamed_barrier(?:_or)?\(([^;]*?)[;{]", text)]
+    assert len(calls) >= 10
+    for name, call in calls:
+        assert re.match(r"1 \+ (wg, 128|G, 128 \* G)[,)]", call), (name, call)
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setenv("FOSCAR_B200_LIB", str(tmp_path / "nope.so"))
