@@ -1096,7 +1096,7 @@ extern "C" int fq_decode(const fq_pools* pools, const fq_decode_args* args, void
   P.q_len = a.q_len > 1 ? a.q_len : 1;
   if (P.q_len > 64) return FQ_ERR_BAD_ARG;
   P.gqa = a.num_qo_heads / pools->num_kv_heads;
-  P.gqa_inv = (65536 + P.gqa - 1) / P.gqa;
+  P.gqa_inv = ((1 << 20) + P.gqa - 1) / P.gqa;
   P.hq = a.num_qo_heads;
   if (P.gqa * P.q_len > 512) return FQ_ERR_TOO_LARGE;   // (column_token's range)
   P.heads_per_kv = P.gqa * P.q_len;

@@ -21,7 +21,7 @@ struct DecodeParams {
   int head_tiles;    // ceil(heads_per_kv / 8)
   int q_len;         // query tokens per request (>= 1)
   int gqa;           // the caller's query heads per KV head
-  int gqa_inv;       // ceil(2^16 / gqa)
+  int gqa_inv;       // ceil(2^20 / gqa)
   int hq;            // the caller's query heads
   int num_items;     // implicit: B*HKV*head_tiles*kv_splits; explicit: row capacity
   int ring_stages;
@@ -34,11 +34,13 @@ struct WorkItem {
   int b, kvh, ht, t0, t1, slot, len, table_off;
 };
 
-// Several query tokens per request (template flag MQ; the one-token builds carry none of it):
-// column hl of KV head kvh is query token hl / gqa, head hl % gqa of the KV head's group. The
-// quotient comes from a multiply and a shift (gqa_inv = ceil(2^16 / gqa), exact for hl < 512).
+// Several query tokens per request (template flag MQ; the one-token builds at head_dim 128 and 256
+// carry none of it): column hl of KV head kvh is query token hl / gqa, head hl % gqa of the KV head's
+// group. The quotient comes from a multiply and a shift, with gqa_inv = ceil(2^20 / gqa): for gqa and
+// hl up to 512 the product exceeds 2^20 hl / gqa by less than 512, hence the quotient by less than
+// 2^-11 < 1 / gqa, and the product stays below 2^30.
 __device__ __forceinline__ int column_token(const DecodeParams& P, int hl) {
-  return (hl * P.gqa_inv) >> 16;
+  return (hl * P.gqa_inv) >> 20;
 }
 
 // (token row, head) of column hl in the caller's q / out / lse / q_descale tensors

@@ -36,7 +36,7 @@ def _case(bits, d, hq, hkv, L, seq, *, kv_splits=None, k_channel=False, graph=Fa
     lse = torch.full((b, L, hq), float("nan"), device="cuda")
     for _ in range(2):      # twice: split units must leave their counters at zero
         out.fill_(float("nan"))
-        w.run(q, cache, out=out, lse=lse, q_descale=qd)
+        w.run(q, cache, out=out, lse=lse if L > 1 else lse.view(b, hq), q_descale=qd)
         torch.cuda.synchronize()
         assert w.last_status() == 0
     pools = cpu_twin(cache, k, v, slots)
@@ -80,6 +80,15 @@ def test_uniform_splits_and_descale(d, kv_splits):
     alone), with q_descale per (request, token, head)."""
     w = _case(4, d, 16, 2, 2, [129, 257, 4097, 700], kv_splits=kv_splits, descale=True, seed=5)
     assert w.kv_splits == kv_splits
+
+
+@pytest.mark.parametrize("d,gqa,L", [(64, 257, 1), (64, 280, 1), (64, 500, 1), (64, 511, 1),
+                                     (64, 512, 1), (128, 512, 1), (256, 300, 1),
+                                     (64, 151, 3), (128, 195, 2), (256, 210, 2), (64, 256, 2)])
+def test_wide_groups(d, gqa, L):
+    """Up to 512 columns a KV head: every column finds its query token and head (a product with a
+    rounded 1 / gqa has to give hl / gqa exactly), in the last request and KV head as well."""
+    _case(4, d, 2 * gqa, 2, L, [5, 130, 70], seed=gqa + L)
 
 
 def test_minimum_length_and_single_request():
