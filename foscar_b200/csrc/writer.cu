@@ -164,9 +164,10 @@ __device__ inline float clip_threshold(const float (&x)[CH], int index) {
 
 // Quantize the CH values of this lane against its group's (s, z) into the lane's part of the
 // row's code words: WPL whole words, or its fields of a word shared with neighbouring lanes.
-// A code is rni(div.rn(x - z, s)). Most are told without a division: the product with 1/s is
-// within 2^-21 of the quotient's fl, so unless it lies within 1e-5 of a half integer (codes are at
-// most 15) both round alike; a warp with such a value, a value outside the envelope or a NaN takes
+// A code is rni(div.rn(x - z, s)). Most are told without a division: 1/s, the product with it and the
+// quotient it stands for are each rounded by at most 2^-24 of themselves, so product and quotient
+// (at most 15) are within 3e-6 of each other, and unless the product lies within 1e-5 of a half
+// integer both round alike; a warp with such a value, a value outside the envelope or a NaN takes
 // the divisions (about one pass in a hundred). The rounding adds 1.5 * 2^23, whose bits are taken
 // off the assembled word once. Called by whole warps. Sixteen values a lane (head_dim 256) divide
 // every value: the short form's registers cost more there than it saves (115 against 107 us on
