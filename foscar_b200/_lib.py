@@ -28,14 +28,6 @@ def tile_tokens(bits: int, head_dim: int) -> int:
     return int(n)
 
 
-def ctas_per_sm(bits: int, head_dim: int) -> int:
-    """CTAs of the decode kernel's build for (bits, head_dim) that share an SM (1 or 2)."""
-    n = load().fq_ctas_per_sm(bits, head_dim)
-    if n < 0:
-        check(n, "ctas_per_sm")
-    return int(n)
-
-
 def piece_overhead(bits: int, head_dim: int) -> int:
     """Fixed cost of a work piece in tile units, as the balanced planner counts it."""
     n = load().fq_piece_overhead(bits, head_dim)

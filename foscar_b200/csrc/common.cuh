@@ -1,6 +1,7 @@
 // Shared device helpers: pool-format arithmetic and sm_100a PTX wrappers (mbarrier, asynchronous
-// copies, tcgen05 tensor-memory and MMA instructions). Every wait is bounded by a cycle budget:
-// when it runs out the waiter raises the CTA's abort flag and the caller's status word and
+// copies, tcgen05 tensor-memory and MMA instructions). Every wait of one role for another is bounded by
+// a cycle budget (barriers, which no budget can end, join whole worker groups or the CTA, whose
+// threads all reach them whatever their waits returned): when it runs out the waiter raises the CTA's abort flag and the caller's status word and
 // falls through, so a protocol error ends the kernel instead of hanging the GPU.
 #pragma once
 #include <cuda_runtime.h>
@@ -75,9 +76,6 @@ constexpr long long WAIT_BUDGET_CYCLES = 2000000000LL;
 // Wait for a barrier phase, bounded. `abort_flag` is a CTA-shared word: once any waiter has
 // given up every later wait returns at once, so the CTA drains in bounded time. The cycle
 // budget of a wait sits two words after the flag (set_wait_budget).
-// `site` names the call site for the optional wait profile (see FQ_WAIT_PROFILE): the cycles
-// lane 0 of each warp spent blocked are summed per site in the words after the budget.
-constexpr int WAIT_SITES = 32;
 __device__ inline void set_wait_budget(volatile int* abort_flag, long long cycles) {
   *reinterpret_cast<volatile long long*>(abort_flag + 2) = cycles;
 }
@@ -98,30 +96,19 @@ static __device__ __noinline__ void mbar_wait_slow(uint32_t bar, uint32_t parity
     }
   }
 }
-#ifndef FQ_WAIT_PROFILE
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity,
-                                          volatile int* abort_flag, int* status, int = -1,
-                                          int* = nullptr) {
+                                          volatile int* abort_flag, int* status) {
   if (!mbar_try(bar, parity)) mbar_wait_slow(bar, parity, abort_flag, status);
 }
-#else
-// Diagnostic build: the cycles each thread spends inside a wait are summed per call site in
-// a thread-local array (constant indices, so it stays in registers).
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity,
-                                          volatile int* abort_flag, int* status, int site = -1,
-                                          int* wprof = nullptr) {
-  const long long t0 = clock64();
-  if (!mbar_try(bar, parity)) mbar_wait_slow(bar, parity, abort_flag, status);
-  if (wprof != nullptr && site >= 0) wprof[site] += static_cast<int>(clock64() - t0);
-}
-#endif
 
-// Bounded wait for a shared-memory word that only grows (a count of events) to reach `want`.
-// One thread polls; the caller follows with a warp or group synchronisation.
+// Bounded wait for a shared-memory word to reach `want` (a count of events, which only grows) or,
+// with AT_LEAST false, to equal it. One thread polls; the caller follows with a warp or group
+// synchronisation.
+template <bool AT_LEAST = true>
 static __device__ __noinline__ void count_wait(volatile int* word, int want,
                                                volatile int* abort_flag, int* status) {
   long long t0 = 0;
-  for (uint32_t tries = 1; *word < want; ++tries) {
+  for (uint32_t tries = 1; AT_LEAST ? *word < want : *word != want; ++tries) {
     if ((tries & 31u) != 0) continue;
     if (*abort_flag) return;
     const long long now = clock64();
@@ -480,7 +467,6 @@ __device__ inline float2 e4m3x2_to_f32x2(uint32_t v) {
   __half2 h = *reinterpret_cast<__half2*>(&h2);
   return __half22float2(h);
 }
-__device__ inline float e4m3_to_f32(uint32_t byte) { return e4m3x2_to_f32x2(byte & 0xFF).x; }
 
 __device__ inline float fast_exp2(float x) {
   float y;

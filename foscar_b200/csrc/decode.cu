@@ -964,13 +964,15 @@ umma_selftest_kernel(int mode, const uint8_t* k_bytes, const uint8_t* q_bytes,
 
 // Wait self test (see foscar_b200.h): every form of wait that the decode kernels' roles use, one
 // after the other, each with the given cycle budget and for something that never comes: a barrier
-// phase that nothing completes, waited for by single threads, and a hand-off that is two of its four
-// arrivals short, waited for by whole warps. The first waiter to run out raises the CTA's abort flag
+// phase that nothing completes, waited for by single threads; a hand-off that is two of its four
+// arrivals short, waited for by whole warps; and a shared-memory word that neither reaches nor equals
+// what one thread of a warp waits for. The first waiter to run out raises the CTA's abort flag
 // and FQ_STATUS_TIMEOUT; the others fall through; the kernel returns.
 __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(long long budget, int* status,
                                                               int* gave_up) {
   __shared__ __align__(8) unsigned long long bar_words[2];
   __shared__ __align__(8) int ctl_words[4];
+  __shared__ int word;
   volatile int* abort_flag = ctl_words;
   const uint32_t alone = smem_u32(&bar_words[0]), handoff = smem_u32(&bar_words[1]);
   if (threadIdx.x == 0) {
@@ -978,6 +980,7 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(long long budget, 
     set_wait_budget(abort_flag, budget);
     mbar_init(alone, 1);
     mbar_init(handoff, 4);
+    word = 1;
     fence_barrier_init();
   }
   __syncthreads();
@@ -994,6 +997,10 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(long long budget, 
   next_form();
   mbar_arrive_elect(handoff);                 // (one a warp: two of four)
   mbar_wait_warp(handoff, 0, abort_flag, status);
+  next_form();
+  if (threadIdx.x % 32 == 0) count_wait<true>(&word, 2, abort_flag, status);
+  next_form();
+  if (threadIdx.x % 32 == 0) count_wait<false>(&word, 0, abort_flag, status);
   next_form();
   if (threadIdx.x == 0 && gave_up != nullptr) *gave_up = all;
 }
@@ -1019,7 +1026,6 @@ template <int BITS, int D, int GP, int KG = 1, bool MQ = false>
 static int launch_decode(DecodeParams& P, cudaStream_t stream) {
   using SP = SmemPlan<BITS, D>;
   constexpr int THREADS = DECODE_THREADS, LIMIT = SMEM_LIMIT;
-  P.ring_stages = SP::NS;
   P.tile_tokens = SP::TT;
   P.wait_budget = P.a.wait_budget_cycles > 0 ? P.a.wait_budget_cycles : WAIT_BUDGET_CYCLES;
   // Shared memory the ring leaves over holds more decoded work items (32 bytes each), up to

@@ -24,7 +24,7 @@ struct DecodeParams {
   int gqa_inv;       // ceil(2^20 / gqa)
   int hq;            // the caller's query heads
   int num_items;     // implicit: B*HKV*head_tiles*kv_splits; explicit: row capacity
-  int ring_stages;
+  int ring_stages;   // (head_dim 256: the other kernels' are fixed when they are built)
   int tile_tokens;   // tile_tokens(bits, head_dim)
   int item_slots;    // work items a CTA keeps decoded in shared memory
   long long wait_budget;   // cycle budget of one device wait
@@ -102,8 +102,7 @@ struct SmemPlan {
   static constexpr int ROW = 128;
   static constexpr int VOP_STAGE = TILE * ROW;   // expanded V operand, one tile
   static constexpr int Q_BYTES = 16 * ROW;             // 16 MMA rows
-  static constexpr int P_BYTES = TT * 16;              // 16 bytes (8 hi + 8 lo) per token, a
-                                                       // plane of 128 rows per token of a lane
+  static constexpr int P_BYTES = TT * 16;              // 16 bytes (8 hi + 8 lo) per token
   static constexpr int VOP_OFF = 0;
   static constexpr int Q_OFF = VOP_OFF + G * VOP_STAGE;
   static constexpr int P_OFF = Q_OFF + 2 * Q_BYTES;
@@ -278,7 +277,8 @@ __device__ inline __half2 e4m3x2_to_f16x2(uint32_t v) {
   return *reinterpret_cast<__half2*>(&r);
 }
 
-// The same with the row given by its swizzled piece 0: piece v sits at `src` xor 16 v.
+// A token's code row as packed words: `src` is the swizzled place of its piece 0, and piece v sits at
+// `src` xor 16 v.
 template <int BITS, int D>
 __device__ __forceinline__ void load_code_row(uint32_t src, uint32_t (&w)[D * BITS / 32]) {
 #pragma unroll
@@ -286,15 +286,6 @@ __device__ __forceinline__ void load_code_row(uint32_t src, uint32_t (&w)[D * BI
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(w[4 * v]), "=r"(w[4 * v + 1]), "=r"(w[4 * v + 2]), "=r"(w[4 * v + 3])
                  : "r"(src ^ (v << 4)));
-}
-// Load this thread's token row (RB bytes at `src`) as packed words.
-template <int BITS, int D>
-__device__ inline void load_row(uint32_t src, uint32_t (&w)[D * BITS / 32], int swz) {
-#pragma unroll
-  for (int v = 0; v < D * BITS / 128; ++v)
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(w[4 * v]), "=r"(w[4 * v + 1]), "=r"(w[4 * v + 2]), "=r"(w[4 * v + 3])
-                 : "r"(src + ((v ^ swz) << 4)));   // chunk v sits at chunk v ^ swz of the row
 }
 // Unpack packed words into exact operand bytes, one per code, in expansion order:
 // out[(8/BITS) * wi + k] = (w[wi] >> (BITS * k)) & mask.

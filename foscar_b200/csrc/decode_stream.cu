@@ -47,6 +47,7 @@ namespace stream {
 
 namespace {
 
+constexpr int D = 64;              // head_dim
 constexpr int CHUNK = 32;          // tokens of a chunk
 // A warp's chunks looked up ahead: a ring of {page id, 2 * KV head + page half}, or {-1, NO_CHUNK}:
 // no such chunk, or nothing valid in it (the page id is the caller's word as it stands, so no value
@@ -60,12 +61,11 @@ constexpr int SLOTS = 32;          // items that may be waiting for their last w
 constexpr float MAX_LAG = 3.f, HEADROOM = 3.f;
 
 // Shared-memory plan. All offsets from a 128-byte aligned base.
-template <int BITS, int D, int GP>
+template <int BITS, int GP>
 struct StreamPlan {
   static constexpr int W = 16;                         // warps
   static constexpr int RB = D * BITS / 8;              // code row bytes
   static constexpr int CHUNKS = RB / 16;               // 16-byte pieces of a row
-  static constexpr int CODE_PAGE = PAGE * RB;
   static constexpr int CODE = CHUNK * RB;              // a chunk's K (or V) codes
   static constexpr int K_OFF = 0, V_OFF = CODE, R_OFF = 2 * CODE;
   static constexpr int STAGE = 2 * CODE + CHUNK * 16;
@@ -73,10 +73,11 @@ struct StreamPlan {
   static constexpr int QR = D / 8;                     // query operand registers
   static constexpr int NST = GP == 4 ? 2 * MT : 4 * MT;   // state registers of a lane
   static constexpr int STATE = NST * 128;              // a warp's O: GP heads x D, f32
+  static_assert(CHUNKS == 1 || CHUNKS == 2, "one piece a row at INT2, two at INT4");
   // 16-byte piece c of ring row r sits at piece c ^ row_swizzle(r): the eight rows an ldmatrix
   // matrix reads at the same piece then fall on different banks
   __host__ __device__ static constexpr int row_swizzle(int row) {
-    return CHUNKS == 8 ? (row & 7) : (CHUNKS == 4 ? (row >> 1) & 3 : (CHUNKS == 2 ? (row >> 2) & 1 : 0));
+    return CHUNKS == 2 ? (row >> 2) & 1 : 0;
   }
   static constexpr int CTL_OFF = 0;                    // abort flag and wait budget, counters
   static constexpr int META_OFF = 512;                 // per warp m, l, c of eight columns
@@ -162,36 +163,18 @@ struct Field {
 };
 
 // Where O^T's rows sit: (m-tile f, row half hi, lane row r) -> channel and field.
-template <int BITS, int D>
+template <int BITS>
 __device__ __forceinline__ int o_field(int f, int hi) {
-  constexpr int NF = Field<BITS>::NF;
-  return D * BITS / 128 == 1 ? 2 * f + hi : f % NF;
+  return BITS == 2 ? 2 * f + hi : f;
 }
-template <int BITS, int D>
+template <int BITS>
 __device__ __forceinline__ int o_channel(int f, int hi, int r) {
   constexpr int NF = Field<BITS>::NF, WC = 32 / BITS;
-  const int piece = D * BITS / 128 == 1 ? r : 8 * (2 * (f / NF) + hi) + r;
-  const int F = (piece & 1) * NF + o_field<BITS, D>(f, hi);
+  const int piece = BITS == 2 ? r : 8 * hi + r;
+  const int F = (piece & 1) * NF + o_field<BITS>(f, hi);
   return WC * (piece >> 1) + F / 2 + (WC / 2) * (F % 2);
 }
 
-// Bounded wait for a word of shared memory to reach (AT_LEAST) or to equal `want`.
-template <bool AT_LEAST>
-__device__ __noinline__ void spin_wait(volatile int* word, int want, volatile int* abort_flag,
-                                       int* status) {
-  long long t0 = 0;
-  for (uint32_t tries = 1; AT_LEAST ? *word < want : *word != want; ++tries) {
-    if ((tries & 31u) != 0) continue;
-    if (*abort_flag) return;
-    const long long now = clock64();
-    if (t0 == 0) t0 = now;
-    if (now - t0 > *reinterpret_cast<volatile long long*>(abort_flag + 2)) {
-      *abort_flag = 1;
-      if (status) atomicOr(status, FQ_STATUS_TIMEOUT);
-      return;
-    }
-  }
-}
 // Bounded wait until a word of shared memory satisfies a condition; all lanes follow lane 0.
 // (the abort flag and the cycle budget sit at the start of the control block)
 template <bool AT_LEAST>
@@ -199,7 +182,7 @@ __device__ __forceinline__ void warp_wait(volatile int* word, int want, volatile
                                           int* status) {
   if ((threadIdx.x & 31) == 0) {
     if (AT_LEAST ? *word < want : *word != want)
-      spin_wait<AT_LEAST>(word, want, abort_flag, status);
+      count_wait<AT_LEAST>(word, want, abort_flag, status);
   }
   __syncwarp();
 }
@@ -207,7 +190,8 @@ __device__ __forceinline__ void warp_wait(volatile int* word, int want, volatile
 // Merge of a split unit's partials by one warp: the arithmetic and slot order of merge_kernel.
 // A lane takes channels lane, lane + 32, ...; the slots' (m, l) pairs are fetched one per lane
 // and handed round by shuffles, the o values eight slots at a time.
-template <int D>
+// (merge_unit_partials, decode.cuh, gives a channel to each of a group's 128 threads; here one warp
+// takes a whole row, so a lane holds two channels.)
 __device__ __noinline__ void merge_unit_warp(const DecodeParams& P, int k, int b, int kvh, int ht,
                                              int h0, int h1) {
   constexpr float LN2 = 0.6931471805599453f;
@@ -228,7 +212,7 @@ __device__ __noinline__ void merge_unit_warp(const DecodeParams& P, int k, int b
       ms[j] = s < k ? __ldcg(P.a.m_partial + s * rows + row) : -INFINITY;
       ls[j] = s < k ? __ldcg(P.a.l_partial + s * rows + row) : 0.f;
     }
-    constexpr int SB = CH > 4 ? 4 : 8;   // slots requested together
+    constexpr int SB = 8;   // slots requested together
     float os[SB][CH];
     auto fetch = [&](int s0) {
 #pragma unroll
@@ -334,18 +318,15 @@ __device__ __noinline__ void bad_page(uint32_t records, int* status) {
 
 }  // namespace
 
-template <int BITS, int D, int GP, int KG>
-__global__ void __launch_bounds__(32 * StreamPlan<BITS, D, GP>::W, 1)
+template <int BITS, int GP, bool HALF>
+__global__ void __launch_bounds__(32 * StreamPlan<BITS, GP>::W, 1)
 stream_decode_kernel(const __grid_constant__ DecodeParams P) {
-  // KG: 1 whole-head K with f32 records, 3 the same with bf16 pairs, 2 two 64-channel K groups
-  static_assert(KG == 1 || KG == 3 || (KG == 2 && D == 128),
-                "K groups of 64 channels at head_dim 128");
-  using SP = StreamPlan<BITS, D, GP>;
+  // HALF: the records are bf16 pairs, not f32
+  using SP = StreamPlan<BITS, GP>;
   using FD = Field<BITS>;
   constexpr int W = SP::W, CHUNKS = SP::CHUNKS, RB = SP::RB, MT = SP::MT;
   constexpr int NT = GP == 4 ? 1 : 2;         // tokens of a lane in a group of sixteen
   constexpr int NG = CHUNK / 16;
-  constexpr int NK = KG == 2 ? 2 : 1;         // K groups of a row
   constexpr float LN2 = 0.6931471805599453f;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem0 = (smem_u32(smem_raw) + 127u) & ~127u;
@@ -433,27 +414,17 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
       const uint8_t* vs = P.p.v_codes + off;
       const uint32_t dst = issue_to;
 #pragma unroll
-      for (int c = 0; c < SP::CODE; c += 512) {
-        // rows advance by 32 / CHUNKS per step: only 128-byte rows change their swizzle with it
-        const uint32_t at = CHUNKS == 8 ? code_lane ^ ((c / 512 & 1) * 64u) : code_lane;
-        cp_async16_stream(dst + SP::K_OFF + c + at, ks + c, stream_policy);
-        cp_async16_stream(dst + SP::V_OFF + c + at, vs + c, stream_policy);
+      for (int c = 0; c < SP::CODE; c += 512) {   // (a step of 16 rows keeps the swizzle)
+        cp_async16_stream(dst + SP::K_OFF + c + code_lane, ks + c, stream_policy);
+        cp_async16_stream(dst + SP::V_OFF + c + code_lane, vs + c, stream_policy);
       }
       const uint8_t* ss = static_cast<const uint8_t*>(P.p.scales) + lane16;
-      if constexpr (KG == 1) {           // 16 bytes a token
+      if constexpr (!HALF) {             // 16 bytes a token
         ss += static_cast<uint64_t>(blk2) * (16 * CHUNK);
         cp_async16_stream(dst + SP::R_OFF + 16 * lane, ss, stream_policy);
-      } else if constexpr (KG == 3) {    // 8 bytes a token
+      } else {                           // 8 bytes a token
         ss += static_cast<uint64_t>(blk2) * (8 * CHUNK);
         if (lane < 16) cp_async16_stream(dst + SP::R_OFF + 16 * lane, ss, stream_policy);
-      } else {                           // a page's 8 bytes of K pairs a token, then 4 of V pairs
-        ss += static_cast<uint64_t>(blk2 >> 1) * (12 * PAGE);
-        const uint32_t half = blk2 & 1u;
-        if (lane < 16)
-          cp_async16_stream(dst + SP::R_OFF + 16 * lane, ss + half * (8 * CHUNK), stream_policy);
-        else if (lane < 24)
-          cp_async16_stream(dst + SP::R_OFF + 16 * lane,
-                            ss + (8 * PAGE - 256) + half * (4 * CHUNK), stream_policy);
       }
     } else if (entry.y != NO_CHUNK) {   // (no chunk: nothing to copy)
       bad_page(issue_to + SP::R_OFF, status);
@@ -478,7 +449,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
 
   float O[MT][4];
   uint32_t qr[SP::QR];
-  float hs[2], hq[2][NK];                     // score scale; sums of the query row (per K group)
+  float hs[2], hq[2];                         // score scale; sum of the query row
   float m[2], l[2], c[2];
   float thr[2];                               // excess that raises m; -inf: no finite score yet
   int lim[2];                                 // the heads' first invisible position
@@ -494,9 +465,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
     const uint8_t* q = static_cast<const uint8_t*>(P.a.q) + qrow * D;
     float scale = live ? P.a.sm_scale * 1.4426950408889634f : 0.f;
     if (live && P.a.q_descale != nullptr) scale *= caller_descale<true>(P, w.b, w.kvh, hl);
-    float sum[NK];
-#pragma unroll
-    for (int i = 0; i < NK; ++i) sum[i] = 0.f;
+    float sum = 0.f;
 #pragma unroll
     for (int cc = 0; cc < CHUNKS; ++cc) {
       constexpr int NB = 32 / BITS / 4;       // 4-byte words of the q bytes against one packed word
@@ -516,7 +485,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
         const float2 a = e4m3x2_to_f32x2(raw[i] & 0xFFFF), b = e4m3x2_to_f32x2(raw[i] >> 16);
         s += (a.x + a.y) + (b.x + b.y);
       }
-      sum[NK == 2 ? cc / (CHUNKS / 2) : 0] += s;
+      sum += s;
 #pragma unroll
       for (int f = 0; f < FD::NF; ++f) {
         // channels of fields f and NF + f
@@ -529,18 +498,13 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
         qr[cc * FD::NF + f] = *reinterpret_cast<const uint32_t*>(&v);
       }
     }
-#pragma unroll
-    for (int i = 0; i < NK; ++i) {
-      sum[i] += __shfl_xor_sync(0xFFFFFFFFu, sum[i], 1);
-      sum[i] += __shfl_xor_sync(0xFFFFFFFFu, sum[i], 2);
-    }
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {             // from the operand's columns to the lane's heads
       // (a code is code * 2^-24: the scores' scale makes up for it, the query sums are divided)
       hs[i] = __shfl_sync(0xFFFFFFFFu, scale, 4 * (h0 + i)) * 16777216.f;
-#pragma unroll
-      for (int k = 0; k < NK; ++k)
-        hq[i][k] = __shfl_sync(0xFFFFFFFFu, sum[k], 4 * (h0 + i)) * (1.f / 16777216.f);
+      hq[i] = __shfl_sync(0xFFFFFFFFu, sum, 4 * (h0 + i)) * (1.f / 16777216.f);
       m[i] = l[i] = c[i] = 0.f;
       thr[i] = -INFINITY;
       lim[i] = (w.t1 > w.t0 ? w.len : 0) -
@@ -678,8 +642,8 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
         for (int i = 0; i < SP::NST / MT; ++i) {
           const int hi = GP == 4 ? (j >> 1) : (i >> 1);
           const float unit =
-              1.f / static_cast<float>(1 << FD::bits_up(o_field<BITS, D>(t, hi)));
-          mine[(h0 + (i & 1)) * D + o_channel<BITS, D>(t, hi, r)] =
+              1.f / static_cast<float>(1 << FD::bits_up(o_field<BITS>(t, hi)));
+          mine[(h0 + (i & 1)) * D + o_channel<BITS>(t, hi, r)] =
               fmaf(st[(SP::NST / MT) * t + i], o_mul * unit, c[i & 1]);
         }
       __syncwarp();
@@ -726,7 +690,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
       k = __shfl_sync(0xFFFFFFFFu, k, 0);
       if (k > 0) {
         __threadfence();
-        merge_unit_warp<D>(P, k, w.b, w.kvh, w.ht, 0, GP);
+        merge_unit_warp(P, k, w.b, w.kvh, w.ht, 0, GP);
       }
     }
   };
@@ -755,49 +719,35 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
 #pragma unroll
     for (int tb = 0; tb < NG; ++tb) {
       const uint32_t ka = sb + SP::K_OFF + tb * 16 * RB;
-      float acc[NK][4];
+      float acc[4];
+      uint32_t kw[CHUNKS][2];                 // a piece's words of tokens r and r + 8
+      if constexpr (CHUNKS == 1) ldsm2(ka + lm_off, kw[0][0], kw[0][1]);
+      else ldsm4(ka + lm_off, kw[0][0], kw[CHUNKS - 1][0], kw[0][1], kw[CHUNKS - 1][1]);
 #pragma unroll
-      for (int cp = 0; cp < (CHUNKS + 1) / 2; ++cp) {
-        uint32_t k0[2], k1[2];                // tokens r and r + 8; pieces 2cp, 2cp + 1
-        if constexpr (CHUNKS == 1) ldsm2(ka + lm_off, k0[0], k1[0]);
-        else ldsm4(ka + (lm_off ^ (32u * cp)), k0[0], k0[1], k1[0], k1[1]);
+      for (int cc = 0; cc < CHUNKS; ++cc) {
+        const uint32_t k0 = kw[cc][0], k1 = kw[cc][1];
+        const uint32_t s0 = k0 >> FD::SHIFT, s1 = k1 >> FD::SHIFT;
 #pragma unroll
-        for (int u = 0; u < (CHUNKS == 1 ? 1 : 2); ++u) {
-          const int cc = 2 * cp + u;
-          const int grp = NK == 2 ? cc / (CHUNKS / 2) : 0;
-          const uint32_t s0 = k0[u] >> FD::SHIFT, s1 = k1[u] >> FD::SHIFT;
-#pragma unroll
-          for (int f = 0; f < FD::NF; f += 2) {
-            const uint32_t a0 = FD::get(k0[u], s0, f), a1 = FD::get(k1[u], s1, f),
-                           a2 = FD::get(k0[u], s0, f + 1), a3 = FD::get(k1[u], s1, f + 1);
-            const uint32_t b0 = qr[cc * FD::NF + f], b1 = qr[cc * FD::NF + f + 1];
-            if (f == 0 && cc % (CHUNKS / NK) == 0) mma_f16_first(acc[grp], a0, a1, a2, a3, b0, b1);
-            else mma_f16(acc[grp], a0, a1, a2, a3, b0, b1);
-          }
+        for (int f = 0; f < FD::NF; f += 2) {
+          const uint32_t a0 = FD::get(k0, s0, f), a1 = FD::get(k1, s1, f),
+                         a2 = FD::get(k0, s0, f + 1), a3 = FD::get(k1, s1, f + 1);
+          const uint32_t b0 = qr[cc * FD::NF + f], b1 = qr[cc * FD::NF + f + 1];
+          if (f == 0 && cc == 0) mma_f16_first(acc, a0, a1, a2, a3, b0, b1);
+          else mma_f16(acc, a0, a1, a2, a3, b0, b1);
         }
       }
       if constexpr (GP == 4) {                // columns 4-7 are idle: their lanes take tokens 8-15
 #pragma unroll
-        for (int k = 0; k < NK; ++k)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const float got = __shfl_xor_sync(0xFFFFFFFFu, acc[k][2 + i], 2);
-            if (upper) acc[k][i] = got;
-          }
+        for (int i = 0; i < 2; ++i) {
+          const float got = __shfl_xor_sync(0xFFFFFFFFu, acc[2 + i], 2);
+          if (upper) acc[i] = got;
+        }
       }
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
         const int tok = 16 * tb + 8 * t + tok0;
-        float sk, zk, sv, sk1, zk1;
-        if constexpr (KG == 2) {
-          uint32_t kr0, kr1, vr;
-          asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(kr0), "=r"(kr1)
-                       : "r"(sb + SP::R_OFF + 8 * tok));
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(vr) : "r"(sb + SP::R_OFF + 8 * CHUNK + 4 * tok));
-          sk = __uint_as_float(kr0 << 16); zk = __uint_as_float(kr0 & 0xFFFF0000u);
-          sk1 = __uint_as_float(kr1 << 16); zk1 = __uint_as_float(kr1 & 0xFFFF0000u);
-          sv = __uint_as_float(vr << 16); zv[tb][t] = __uint_as_float(vr & 0xFFFF0000u);
-        } else if constexpr (KG == 1) {
+        float sk, zk, sv;
+        if constexpr (!HALF) {
           asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
                        : "=f"(sk), "=f"(zk), "=f"(sv), "=f"(zv[tb][t])
                        : "r"(sb + SP::R_OFF + 16 * tok));
@@ -812,8 +762,7 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
         wsc[tb][t] = fminf(sv * p2lp, 8000.f);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          float s = fmaf(sk, acc[0][2 * t + i], zk * hq[i][0]);
-          if constexpr (KG == 2) s = fmaf(sk1, acc[NK - 1][2 * t + i], fmaf(zk1, hq[i][NK - 1], s));
+          const float s = fmaf(sk, acc[2 * t + i], zk * hq[i]);
           x[tb][t][i] = fmaf(hs[i], s, -m[i]);
         }
       }
@@ -894,17 +843,14 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
           mma_f16(O[f], FD::get(v0, s0, 2 * f), FD::get(v0, s0, 2 * f + 1), FD::get(v1, s1, 2 * f),
                   FD::get(v1, s1, 2 * f + 1), b0, b1);
       } else {
+        uint32_t v0, v1, v2, v3;
+        ldsm4_t(va + lm_off, v0, v1, v2, v3);
+        const uint32_t s0 = v0 >> FD::SHIFT, s1 = v1 >> FD::SHIFT, s2 = v2 >> FD::SHIFT,
+                       s3 = v3 >> FD::SHIFT;
 #pragma unroll
-        for (int cp = 0; cp < CHUNKS / 2; ++cp) {
-          uint32_t v0, v1, v2, v3;
-          ldsm4_t(va + (lm_off ^ (32u * cp)), v0, v1, v2, v3);
-          const uint32_t s0 = v0 >> FD::SHIFT, s1 = v1 >> FD::SHIFT, s2 = v2 >> FD::SHIFT,
-                         s3 = v3 >> FD::SHIFT;
-#pragma unroll
-          for (int f = 0; f < FD::NF; ++f)
-            mma_f16(O[cp * FD::NF + f], FD::get(v0, s0, f), FD::get(v1, s1, f), FD::get(v2, s2, f),
-                    FD::get(v3, s3, f), b0, b1);
-        }
+        for (int f = 0; f < MT; ++f)
+          mma_f16(O[f], FD::get(v0, s0, f), FD::get(v1, s1, f), FD::get(v2, s2, f),
+                  FD::get(v3, s3, f), b0, b1);
       }
     }
     sb += SP::STAGE;
@@ -915,11 +861,9 @@ stream_decode_kernel(const __grid_constant__ DecodeParams P) {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <int BITS, int GP, int KG>
+template <int BITS, int GP, bool HALF>
 static int launch(DecodeParams& P, cudaStream_t stream) {
-  constexpr int D = 64;
-  using SP = StreamPlan<BITS, D, GP>;
-  P.ring_stages = SP::S;
+  using SP = StreamPlan<BITS, GP>;
   P.tile_tokens = tile_tokens(BITS, D);
   P.wait_budget = P.a.wait_budget_cycles > 0 ? P.a.wait_budget_cycles : WAIT_BUDGET_CYCLES;
   // Shared memory the rings leave over holds more decoded work items (32 bytes each)
@@ -928,7 +872,7 @@ static int launch(DecodeParams& P, cudaStream_t stream) {
   constexpr int smem = SP::MORE_OFF + more * 32 + 128;
   static_assert(smem <= SMEM_LIMIT, "shared-memory plan");
   static bool configured[64] = {};  // per instantiation and device
-  auto kernel = stream_decode_kernel<BITS, D, GP, KG>;
+  auto kernel = stream_decode_kernel<BITS, GP, HALF>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !configured[dev]) {
@@ -961,11 +905,11 @@ static int launch(DecodeParams& P, cudaStream_t stream) {
 int launch_decode_stream(DecodeParams& P, int columns, cudaStream_t s) {
   const bool two = P.p.bits == 2, half = P.p.scale_bf16 != 0;
   if (columns <= 4) {
-    if (two) return half ? stream::launch<2, 4, 3>(P, s) : stream::launch<2, 4, 1>(P, s);
-    return half ? stream::launch<4, 4, 3>(P, s) : stream::launch<4, 4, 1>(P, s);
+    if (two) return half ? stream::launch<2, 4, true>(P, s) : stream::launch<2, 4, false>(P, s);
+    return half ? stream::launch<4, 4, true>(P, s) : stream::launch<4, 4, false>(P, s);
   }
-  if (two) return half ? stream::launch<2, 8, 3>(P, s) : stream::launch<2, 8, 1>(P, s);
-  return half ? stream::launch<4, 8, 3>(P, s) : stream::launch<4, 8, 1>(P, s);
+  if (two) return half ? stream::launch<2, 8, true>(P, s) : stream::launch<2, 8, false>(P, s);
+  return half ? stream::launch<4, 8, true>(P, s) : stream::launch<4, 8, false>(P, s);
 }
 
 }  // namespace fq

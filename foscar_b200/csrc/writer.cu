@@ -55,15 +55,6 @@ __device__ inline long long slot_of(const WriterArgs& a, int token) {
   return static_cast<long long>(page) * PAGE + pos;
 }
 
-__device__ inline float warp_group_min(float x, int lanes) {
-  for (int o = lanes >> 1; o > 0; o >>= 1) x = fminf(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
-  return x;
-}
-__device__ inline float warp_group_max(float x, int lanes) {
-  for (int o = lanes >> 1; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
-  return x;
-}
-
 // Bytes of one (page, head) scale block and where a token's records sit in it.
 __device__ inline long long scale_block_bytes(const fq_pools& p) {
   const int esz = p.scale_bf16 ? 2 : 4;
@@ -72,17 +63,9 @@ __device__ inline long long scale_block_bytes(const fq_pools& p) {
   return static_cast<long long>(elems) * esz;
 }
 
-// Move one cell's count in the table when the cell went from `old` to `now`.
-__device__ inline void settle_count(uint32_t* hist, uint32_t old, uint32_t now) {
-  const bool c_old = (old & 0x7FFFFFFFu) != 0, c_new = (now & 0x7FFFFFFFu) != 0;
-  const uint32_t b_old = vmax_bucket(old), b_new = vmax_bucket(now);
-  if (c_old && c_new && b_old == b_new) return;
-  if (c_new) atomicAdd(hist + b_new, 1u);
-  if (c_old) atomicAdd(hist + b_old, 0xFFFFFFFFu);
-}
-
-// The same into a block-local table of signed deltas (flushed once per block): the pool's counts
-// live in a handful of bins, and a global atomic per raised cell serialises on those addresses.
+// Move one cell's count in the table when the cell went from `old` to `now`: in a block-local table of
+// signed deltas (flushed once per block), since the pool's counts live in a handful of bins, and a
+// global atomic per raised cell serialises on those addresses.
 __device__ inline void settle_count_local(int* local, uint32_t old, uint32_t now) {
   const bool c_old = (old & 0x7FFFFFFFu) != 0, c_new = (now & 0x7FFFFFFFu) != 0;
   const uint32_t b_old = vmax_bucket(old), b_new = vmax_bucket(now);
