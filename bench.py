@@ -78,7 +78,7 @@ def algorithmic_bytes(cfg, seq):
 # DRAM bytes (read + write) of one decode launch of the named workload, from a separate ncu
 # capture of this command at its default arguments (not a figure of this run): reported as
 # `traffic` only when the run's arguments are those of the capture.
-CAPTURED_TRAFFIC = {"c2": 402_309_888, "c2-int4": 717_094_656, "c5-int2": 2_161_422_448,
+CAPTURED_TRAFFIC = {"c2": 397_668_096, "c2-int4": 713_786_368, "c5-int2": 2_157_171_456,
                     "c4": 443_171_840}
 
 

@@ -32,8 +32,10 @@ extern "C" int64_t fq_workspace_bytes(int32_t max_splits, int32_t batch, int32_t
 }
 
 // Fixed cost of a piece in tile units (pipeline refill, the merge of the warps' or groups' states and
-// the output). Swept on B200 (6, 10, 14, 20, 28): at head_dim 128 six to fourteen are within 1 to 2 %; at head_dim 64, where a tile is half the bytes a token and an item ends in one warp's
-// merge, 256 requests of 64-131072 tokens took 652, 568, 521, 509 and 546 us; head_dim 256 as before.
+// the output). Swept on B200 (6, 10, 14, 20, 28): at head_dim 128 six to fourteen are within 1 to 2 %;
+// at head_dim 64, where a tile is half the bytes a token and an item ends in one warp's merge, 256
+// requests of 64-131072 tokens (INT2, eight columns; the one workload swept) took 652, 568, 521, 509
+// and 546 us.
 static long long piece_overhead(int bits, int head_dim) {
   long long ovh = head_dim == 64 ? 20 : (bits == 4 && head_dim == 128 ? 10 : 14);
   if (const char* env = getenv("FOSCAR_B200_PIECE_OVERHEAD")) {   // tuning knob for experiments

@@ -35,10 +35,11 @@
 // elect.sync inside one asm block, ring stages and barriers sit at compile-time offsets, and values
 // that are the same in a warp are told to the compiler (uniform()), because tensor-memory, barrier
 // and descriptor operands have to be in uniform registers. A tile took 1930 warp instructions with
-// lane-0 branches and run-time offsets and takes 1490; on one box 32 requests of 4K-32K tokens (INT2,
-// 32/8 heads) went from 107.8 to 97.4 us, 16 requests of 16K with two query tokens from 66.7 to
-// 55.7. Three, five and six groups measure the same or slower (the registers they cost), and so does one MMA in place of a
-// chain of four: what is left is the instructions' own latency at five warps a scheduler.
+// lane-0 branches and run-time offsets and takes 1575; on one box 32 requests of 4K-32K tokens (INT2,
+// 32/8 heads) went from 107.7 to 98.9 us, 16 requests of 8K-16K with two query tokens from 67.8 to
+// 57.4. Three, five and six groups measure the same or slower (the registers they cost), and so does
+// one MMA in place of a chain of four: what is left is the instructions' own latency at five warps a
+// scheduler.
 // Every role walks the same list of work items, so the pipeline never drains inside an item.
 // Byte-expansion yields channels in a fixed permuted order; Q is loaded in that order and O is
 // stored through it, so no per-element fix-up exists anywhere.
@@ -90,8 +91,6 @@ struct Bars {
 };
 // Named barriers: 0 the CTA, 1 .. G inside a group, 1 + G all groups.
 
-// Tensor-memory column plan (f32 columns): per worker group one K operand stage (a 128-byte row
-// per lane), one S buffer and one O buffer of 16 columns.
 // INT2 with whole-head K at head_dim 128: the K rows are unpacked like the V rows, at five instead
 // of seven instructions a packed word (odd operand words hold 4 * code), and the idle half of the
 // sixteen query rows takes the odd words' products into score columns 8-15.
@@ -99,6 +98,8 @@ __host__ __device__ constexpr bool odd_columns(int bits, int head_dim, int kg) {
   return bits == 2 && head_dim == 128 && kg != 2;
 }
 
+// Tensor-memory column plan (f32 columns): per worker group one K operand stage (a 128-byte row
+// per lane), one S buffer and one O buffer of 16 columns.
 template <int BITS, int D>
 struct TmemPlan {
   static constexpr int G = WORKER_GROUPS;

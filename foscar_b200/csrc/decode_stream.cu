@@ -31,7 +31,8 @@
 // tokens at head_dim 128, 16 at head_dim 64, while softmax and hand-offs cost the same. Measured,
 // start of either form against the other: 256 requests of 64-131072 tokens (INT2, 64/8 heads x 64)
 // 517 us here and 595 us with tcgen05; at head_dim 128 32 requests of 4K-32K tokens (INT2) 115 and
-// 97 us.
+// 97 us. Against the tcgen05 form's last build here one request of 4000 tokens (64/8 heads) takes 19.7
+// us (18.3), 16 of 2000-16000 37.8 (45.0), 64 of 16384 132 (174).
 //
 // A work item ends with the warps' states (m, l, c, O) merged in the order of its first chunks'
 // warps: each leaves its state in its shared-memory slot, counts itself in and goes on with its
