@@ -35,7 +35,7 @@
 // elect.sync inside one asm block, ring stages and barriers sit at compile-time offsets, and values
 // that are the same in a warp are told to the compiler (uniform()), because tensor-memory, barrier
 // and descriptor operands have to be in uniform registers. A tile took 1930 warp instructions with
-// lane-0 branches and run-time offsets and takes 1575; on one box 32 requests of 4K-32K tokens (INT2,
+// lane-0 branches and run-time offsets and takes 1575; side by side 32 requests of 4K-32K tokens (INT2,
 // 32/8 heads) went from 107.7 to 98.9 us, 16 requests of 8K-16K with two query tokens from 67.8 to
 // 57.4. Three, five and six groups measure the same or slower (the registers they cost), and so does
 // one MMA in place of a chain of four: what is left is the instructions' own latency at five warps a
